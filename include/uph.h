@@ -212,19 +212,20 @@ uph_status uph_sim_set_graph(uph_sim *sim, int32_t steps_per_graph);
  * corrector is sph.cc:137-168.) */
 uph_status uph_sim_set_fused_step(uph_sim *sim, int32_t enable);
 
-/* Whether the rate passes keep a candidate list per fluid particle between
- * cell-list builds (default 1): at a build's first pass each particle lists
- * the records of its tile's block within the search radius plus twice the
- * largest displacement before the next build (up to 24 of them), and the
- * passes until the next build test only those instead of walking the cell
- * stencil.  The pairs, their order and so the results are bit-identical
- * either way.  (The reference rebuilds its kd-tree search every call,
- * Search.cc:5-44.) */
+/* Whether a step's pass keeps a candidate list per fluid particle between
+ * cell-list builds (default 1): after a build each particle lists the records
+ * of its tile's block within the search radius plus the largest distance two
+ * particles can close before the next build (up to 32 of them at h = 1.3 dx,
+ * more for wider kernels), and the passes until the next build test only
+ * those.  With 0 every step lists them afresh from the cell stencil.  The
+ * pairs, their order and so the results are bit-identical either way.  (The
+ * reference rebuilds its kd-tree search every call, Search.cc:5-44.) */
 uph_status uph_sim_set_candidate_lists(uph_sim *sim, int32_t enable);
 
 /* Execution tuning (no counterpart in the reference): cell width = search
- * radius / reach (reach 1-3), particle-storage tile edge in cells (power of
- * two <= 32) and the storage re-sort interval in steps.  Defaults 2, 8, 16. */
+ * radius / reach (reach 1-3), particle-storage tile edge in cells (tile +
+ * 2 reach <= 32) and the storage re-sort interval in steps.  Defaults 2, 11
+ * (5 and 7 for tanks of up to 15,000 and 30,000 particles in FP64), 64. */
 uph_status uph_sim_set_tuning(uph_sim *sim, int32_t reach, int32_t tile, int32_t reorder_interval);
 
 /* Picks the tuning by timing `trial_steps` steps per candidate on this

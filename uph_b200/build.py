@@ -29,13 +29,14 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + INCLUD
 
 # (source, extra flags).  The leapfrog and the wall laws (leapfrog.cuh) are
 # compiled without multiply-add contraction so their arithmetic rounds
-# exactly like the reference's; the REF pass applies the leapfrog in its
-# epilogue, and its own pair arithmetic names every fused multiply-add.
+# exactly like the reference's; the rate passes apply the leapfrog in their
+# epilogues, and their pair arithmetic names every fused multiply-add, so that
+# every kernel a pass is instantiated in rounds alike.
 CORE_SOURCES = [
     ("host.cpp", []),
     ("celllist.cu", []),
     ("ref_pass.cu", ["--fmad=false"]),
-    ("wcsph_pass.cu", []),
+    ("wcsph_pass.cu", ["--fmad=false"]),
     ("integrate.cu", ["--fmad=false"]),
     ("virtual.cu", ["--fmad=false"]),
     ("sim.cu", []),

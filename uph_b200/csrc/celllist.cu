@@ -192,9 +192,12 @@ __global__ void __launch_bounds__(kCellBuildThreads) k_cell_build(const CellBuil
     if (A.step_counter) *A.step_counter += 1;
   }
   // the list from the last build is still complete: nothing to do (every
-  // block reads the flag before any block can clear it, in phase 4)
+  // block reads the flag before any block can clear it, after the barriers)
   if (A.rebuild && *(volatile unsigned *)A.rebuild == 0u) return;
-  cell_build_phases(A, s_off, s_wt);
+  if (cell_build_phases(A, BarrierPhases{A.G.bar, A.err}, s_off, s_wt) && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (A.rebuild) *A.rebuild = 0u;
+    if (A.G.gen) *A.G.gen += 1u;  // the passes' candidate lists and recorded tiles are stale
+  }
 }
 
 uph_status launch_cell_build(const DevParams &P, const double *x, const double *y, int first, int count,
@@ -217,19 +220,9 @@ uph_status launch_cell_build(const DevParams &P, const double *x, const double *
   const int want = std::max((count + kCellBuildThreads - 1) / kCellBuildThreads,
                             (G.ncell + 4 * kCellBuildThreads - 1) / (4 * kCellBuildThreads));
   const int blocks = std::max(1, std::min(mb, want));
-  CellBuildArgs A;
-  A.P = P;
-  A.x = x;
-  A.y = y;
-  A.first = first;
-  A.count = std::max(count, 0);
-  A.G = G;
-  A.err = err;
-  A.storage_order = storage_order ? 1 : 0;
-  A.rebuild = check_rebuild ? P.rebuild : nullptr;
-  A.xbin = P.xbin;
-  A.ybin = P.ybin;
-  A.stats = stats ? *stats : PassStats{nullptr, nullptr};
+  CellBuildArgs A = cell_build_args(P, x, y, first, count, G, err, storage_order);
+  if (check_rebuild) A.rebuild = P.rebuild;
+  if (stats) A.stats = *stats;
   A.step_counter = step_counter;
   A.dyn_count = dyn_count;
   cudaLaunchConfig_t cfg = {};

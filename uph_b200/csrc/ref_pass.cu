@@ -56,12 +56,25 @@
 // the expensive loop.
 #include <limits.h>
 
+#include "cell_build.cuh"
 #include "leapfrog.cuh"
-#include "tile_pass.cuh"
+#include "tile_stream.cuh"
 
 namespace uph {
 
+// The sums over a particle's pairs, without the factors every pair shares:
+// the terms in the kernel gradient without its normalisation
+// (DevParams::dw_alpha_h2), those in W without w_alpha.
+//   dp   = P_a/rho_a drho   + kappa P_a dpd
+//   dp_a = P_a/rho_a dpa_v  + kappa P_a dpa_d
+// ref_finish applies them.
 struct RefAcc {
+  double drho, dpd, ax, ay;
+  double drho_a, dpa_v, dpa_d, ax_a, ay_a;
+  double frho, fp, fu, fv;
+};
+// the rates of one particle
+struct RefRates {
   double drho, dp, ax, ay;
   double drho_a, dp_a, ax_a, ay_a;
   double frho, fp, fu, fv;
@@ -69,7 +82,8 @@ struct RefAcc {
 
 // wall forces of a listed pair whose i side is this fluid particle
 __device__ __forceinline__ void wall_pair_force(const DevParams &P, int itb, double r2, double dxa, double dya,
-                                                double dua, double dva, double ma, RefAcc &A)
+                                                double dua, double dva, double ma, double &ax, double &ay,
+                                                double &ax_a, double &ay_a)
 {
   const double r = sqrt(r2);
   double sx = 0.0, sy = 0.0;
@@ -84,11 +98,11 @@ __device__ __forceinline__ void wall_pair_force(const DevParams &P, int itb, dou
       sy = -c1 * dya - c2 * dya;
     }
   }
-  A.ax_a += sx;
-  A.ay_a += sy;
+  ax_a += sx;
+  ay_a += sy;
   if (P.boundary_force == 3) {
-    A.ax += sx;
-    A.ay += sy;
+    ax += sx;
+    ay += sy;
   } else if (P.boundary_force == 4 && (itb == 2 || itb == 3) && r < P.dx) {
     // ImprovedMonaghan, derivatives.c:1955-2012
     const double hh = P.h;
@@ -102,29 +116,31 @@ __device__ __forceinline__ void wall_pair_force(const DevParams &P, int itb, dou
     const double rd = r - P.dx / 5.0;
     const double vmax = P.mach_c * P.mach_c / 5.0;
     const double c = vmax * phi / (rd * r);
-    A.ax += c * dxa;
-    A.ay += c * dya;
+    ax += c * dxa;
+    ay += c * dya;
   } else if (P.boundary_force == 5 && itb == 2 && r < P.dx) {
     // SerialSpringBoundaryForces, derivatives.c:2452-2479
-    A.ax -= (P.k_spring * dxa + P.c_damp * dua) / ma;
-    A.ay -= (P.k_spring * dya + P.c_damp * dva) / ma;
+    ax -= (P.k_spring * dxa + P.c_damp * dua) / ma;
+    ay -= (P.k_spring * dya + P.c_damp * dva) / ma;
   }
 }
 
 // ---- partner records -----------------------------------------------------------
-// One particle's fields as the pair loop reads them: the SoA state plus the
-// per-particle factors every pair would otherwise recompute (Tait's
-// rho0 c0^2 + gamma p, 1/rho^2, rhot/rho, m/rho).  144 bytes, read as nine
-// 16-byte shared-memory loads.
+// One particle's fields as the pair loop reads them, as they stand in the
+// state arrays: 112 bytes, read as seven 16-byte shared-memory loads.
+// Factors such as Tait's rho0 c0^2 + gamma p or 1/rho^2 are formed per pair
+// (four operations of about 105): kept in the record they would make it
+// 144 bytes, and the stream's two buffers (tile_stream.cuh) would not hold a
+// tile's block.
 // (The listing's FP32 positions, relative to the CTA's block origin, are a
 // separate shared-memory array: the pair loop never reads them.)
 struct __align__(16) RefRec {
-  double x, y, u, v, ut, vt, rho, rhot, p, pt, m, ir, irt, P, ir2, C, V;
+  double x, y, u, v, ut, vt, rho, rhot, p, pt, m, irt, ir;
   int orig, itype;
 };
-static_assert(sizeof(RefRec) == 144, "RefRec is nine 16-byte chunks");
+static_assert(sizeof(RefRec) == 112, "RefRec is seven 16-byte chunks");
 
-__device__ __forceinline__ RefRec load_ref_rec(const DevParams &P, const SlotArrays &S, int s)
+__device__ __forceinline__ RefRec load_ref_rec(const SlotArrays &S, int s)
 {
   RefRec r;
   r.x = S.x[s];
@@ -138,12 +154,8 @@ __device__ __forceinline__ RefRec load_ref_rec(const DevParams &P, const SlotArr
   r.p = S.p[s];
   r.pt = S.pt[s];
   r.m = S.m[s];
-  r.ir = S.inv_rho[s];
   r.irt = S.inv_rhot[s];
-  r.P = fma(P.gamma, r.p, P.rho0c2);
-  r.ir2 = r.ir * r.ir;
-  r.C = r.rhot * r.ir;
-  r.V = r.m * r.ir;
+  r.ir = S.inv_rho[s];
   r.orig = S.orig[s];
   r.itype = S.itype[s];
   return r;
@@ -152,55 +164,61 @@ __device__ __forceinline__ RefRec load_ref_rec(const DevParams &P, const SlotArr
 // The particle a thread owns, with its per-particle constants.
 struct RefOwn {
   RefRec r;
-  double IPa;  // P_a / rho_a
-  double G4a;  // 4 gamma kappa P_a
-  double KPa;  // kappa P_a
+  double PR;   // P_a + rho0 c0^2, so that P_a + P_b = PR + gamma p_b
+  double ir2;  // 1 / rho_a^2
   double A1a;  // p_a / rho_a^2
+  double C;    // rhot_a / rho_a
 };
 
 __device__ __forceinline__ RefOwn make_own(const DevParams &P, const RefRec &r)
 {
   RefOwn o;
   o.r = r;
-  o.IPa = r.ir * r.P;
-  o.G4a = 4.0 * (P.gamma * P.kappa) * r.P;
-  o.KPa = P.kappa * r.P;
-  o.A1a = r.p * r.ir2;
+  o.PR = fma(P.gamma, r.p, P.rho0c2) + P.rho0c2;
+  o.ir2 = r.ir * r.ir;
+  o.A1a = r.p * o.ir2;
+  o.C = r.rhot * r.ir;
   return o;
 }
 
 // The per-a sums of one pair (a, b), a = the own particle.  With
 // g = F (x_a - x_b) and the header's formulas, rearranged so that the pair
-// shares one reciprocal and per-particle factors come from the records:
+// shares one reciprocal and factors common to a particle's pairs are applied
+// once, to the sums (RefAcc):
 //   1 / (r^2 + 0.01 h^2), 1 / (P_a + P_b) and 1 / (1/rho_a + 1/rho_b)
 //   all from rr = 1 / ((r^2 + 0.01 h^2)(P_a + P_b)(1/rho_a + 1/rho_b));
 //   (x_a - x_b) . g = F r^2;
+//   gamma kappa dp 4P_a/(P_a + P_b) - kappa P_a drho Sr
+//     = kappa P_a (4 gamma dp / (P_a + P_b) - drho Sr);
 //   S . g = -F r^2 (v_a - v_b) for the deviatoric S of the viscous terms
 //   (its terms in dx dy dv cancel exactly), so both viscous forces are
 //   multiples of (v_a - v_b).
-__device__ __forceinline__ void ref_pair(const DevParams &P, const RefOwn &a, const RefRec &b, bool isI, RefAcc &A)
+// About 105 FP64 operations.
+// wall: the pair's wall force acts (i side fluid, partner a wall).
+// kMasked: a pair that is not `on` contributes zeros (both kernels hold a
+// power of t as a factor) instead of being branched around.
+template <bool kMasked>
+__device__ __forceinline__ void ref_pair(const DevParams &P, const RefOwn &a, const RefRec &b, double dxa, double dya,
+                                         double r2, bool isI, bool on, bool wall, RefAcc &A)
 {
-  const double dxa = a.r.x - b.x, dya = a.r.y - b.y;
-  const double r2 = exact_r2(dxa, dya);
   // poly-7 convolution W and deconvolution gradient factor, functions of q^2
   const double q2 = r2 * P.inv_h2;
-  const double t = fma(-0.25, q2, 1.0);
+  const double t = kMasked && !on ? 0.0 : fma(-0.25, q2, 1.0);
   const double t2 = t * t, t4 = t2 * t2;
   const double t7 = t4 * t2 * t, t8 = t4 * t4;
   const double pp = fma(fma(fma(fma(fma(fma(305.0, q2, -628.0), q2, 1184.0), q2, -1984.0), q2, 2816.0), q2, -3072.0), q2, 2048.0);
   const double pp7 = fma(fma(fma(fma(fma(fma(305.0, q2, -1106.0), q2, 1912.0), q2, -2912.0), q2, 3712.0), q2, -3584.0), q2, 2048.0);
-  const double W = P.w_alpha * t8 * pp;
-  const double F = P.dw_alpha_h2 * t7 * pp7;
-  const double Fr2 = F * r2;
+  const double W = t8 * pp;
+  const double F = t7 * pp7;
 
   const double De = r2 + P.eta2;
-  const double SP = a.r.P + b.P;
+  const double SP = fma(P.gamma, b.p, a.PR);
   const double Sr = a.r.ir + b.ir;
   const double SPSr = SP * Sr;
   const double rr = rcp_nr(De * SPSr);
-  const double inv_r2e = rr * SPSr;
-  const double invSP = rr * (De * Sr);
-  const double nu = Fr2 * inv_r2e;
+  const double T = rr * (F * r2);
+  const double nu = T * SPSr;
+  const double g4SP = (rr * (De * Sr)) * P.gamma4;  // 4 gamma / (P_a + P_b)
 
   const double dux = a.r.u - b.u, duy = a.r.v - b.v;
   const double eux = a.r.u - b.ut, euy = a.r.v - b.vt;
@@ -216,28 +234,27 @@ __device__ __forceinline__ void ref_pair(const DevParams &P, const RefOwn &a, co
   A.drho_a = fma(ms * F, Pd, A.drho_a);
   // predictor pressure (PredictingDynamicPressureEquation)
   const double dpp = a.r.p - b.p, dr = a.r.rho - b.rho;
-  const double brk = fma(-(a.KPa * dr), Sr, a.G4a * dpp * invSP);
-  A.dp_a = fma(mbF * a.IPa, Vd, A.dp_a);
-  A.dp_a = fma(ms * b.ir * nu, brk, A.dp_a);
+  const double irnu = b.ir * nu;
+  A.dpa_v = fma(mbF, Vd, A.dpa_v);
+  A.dpa_d = fma(ms * irnu, fma(-dr, Sr, dpp * g4SP), A.dpa_d);
   // fluctuations
-  const double VW = b.V * W;
+  const double VW = (b.m * b.ir) * W;
   A.frho = fma(-VW, dr, A.frho);
   A.fp = fma(-VW, dpp, A.fp);
   const double cfv = isI ? fma(a.r.m, b.irt, -(b.m * a.r.irt)) * W : 0.0;
   A.fu = fma(dux, cfv, A.fu);
   A.fv = fma(duy, cfv, A.fv);
-  // continuity (DensityEquation)
-  const double VrF = b.V * b.rhot * F;
-  A.drho = fma(VrF, Ed, A.drho);
+  // continuity (DensityEquation): V_b rhot_b = m_b rhot_b / rho_b
+  const double Cb = b.rhot * b.ir;
+  A.drho = fma(Cb * mbF, Ed, A.drho);
   // rate-form Tait with diffusion (DynamicPressureEquation)
   const double dpt = a.r.p - b.pt, drt = a.r.rho - b.rhot;
-  const double brk2 = fma(-(a.KPa * drt), Sr, a.G4a * dpt * invSP);
-  A.dp = fma(VrF * a.IPa, Ed, A.dp);
-  A.dp = fma(b.V * nu, brk2, A.dp);
+  A.dpd = fma(b.m * irnu, fma(-drt, Sr, dpt * g4SP), A.dpd);
   // pressure gradients (PredictingPressureGradientForce, PressureGradientForce)
-  const double A1b = b.p * b.ir2;
+  const double ir2b = b.ir * b.ir;
+  const double A1b = b.p * ir2b;
   const double c1 = mbF * (a.A1a + A1b);
-  const double c2 = mbF * fma(a.A1a, b.C, A1b * a.r.C);
+  const double c2 = mbF * fma(a.A1a, Cb, A1b * a.C);
   A.ax_a = fma(-c1, dxa, A.ax_a);
   A.ay_a = fma(-c1, dya, A.ay_a);
   A.ax = fma(-c2, dxa, A.ax);
@@ -247,27 +264,58 @@ __device__ __forceinline__ void ref_pair(const DevParams &P, const RefOwn &a, co
   // stressType 2 keeps the single-step predictor; its corrector force is
   // added after the pass (launch_viscous_two_step)
   if (P.stress_type == 1 || P.stress_type == 2) {
-    const double vis = b.m * P.two_mu0 * rr * SP * Fr2;
-    const double vp = vis * (a.r.ir2 + b.ir2);
+    const double vis = (b.m * P.two_mu0) * (T * SP);
+    const double vp = vis * (a.ir2 + ir2b);
     A.ax_a = fma(-vp, dux, A.ax_a);
     A.ay_a = fma(-vp, duy, A.ay_a);
     if (P.stress_type == 1) {
-      const double D = fma(b.C, a.r.ir2, -(a.r.C * b.ir2));
+      const double D = fma(Cb, a.ir2, -(a.C * ir2b));
       const double sv = (isI ? vis : -vis) * D;
       A.ax = fma(-sv, dux, A.ax);
       A.ay = fma(-sv, duy, A.ay);
     }
   }
-  // wall forces: only pairs whose i is this fluid particle
-  if (isI && a.r.itype == 1 && b.itype >= 2) wall_pair_force(P, b.itype, r2, dxa, dya, dux, duy, a.r.m, A);
+  // wall forces: only pairs whose i is this fluid particle (divided by the
+  // factor ref_finish applies to the pair sums)
+  if (wall) {
+    double wx = 0.0, wy = 0.0, wxa = 0.0, wya = 0.0;
+    wall_pair_force(P, b.itype, r2, dxa, dya, dux, duy, a.r.m, wx, wy, wxa, wya);
+    const double k = 1.0 / P.dw_alpha_h2;
+    A.ax = fma(k, wx, A.ax);
+    A.ay = fma(k, wy, A.ay);
+    A.ax_a = fma(k, wxa, A.ax_a);
+    A.ay_a = fma(k, wya, A.ay_a);
+  }
+}
+
+// the common factors applied to a particle's sums; (bx, by): the wall modes
+// that act on every boundary particle
+__device__ __forceinline__ RefRates ref_finish(const DevParams &P, const RefOwn &o, const RefAcc &A, double bx, double by)
+{
+  const double g = P.dw_alpha_h2, w = P.w_alpha;
+  const double Pa = fma(P.gamma, o.r.p, P.rho0c2);
+  const double IPa = o.r.ir * Pa, KPa = P.kappa * Pa;
+  RefRates R;
+  R.drho = g * A.drho;
+  R.dp = g * fma(IPa, A.drho, KPa * A.dpd);
+  R.ax = fma(g, A.ax, bx);
+  R.ay = fma(g, A.ay, by);
+  R.drho_a = g * A.drho_a;
+  R.dp_a = g * fma(IPa, A.dpa_v, KPa * A.dpa_d);
+  R.ax_a = g * A.ax_a;
+  R.ay_a = g * A.ay_a;
+  R.frho = w * A.frho;
+  R.fp = w * A.fp;
+  R.fu = w * A.fu;
+  R.fv = w * A.fv;
+  return R;
 }
 
 // gravity, sponge, Tait pressure, stores
 __device__ __forceinline__ void ref_epilogue(const DevParams &P, const SlotArrays &S, int a, const RefOwn &o,
-                                             RefAcc &A, double bx, double by)
+                                             const RefAcc &sums, double bx, double by)
 {
-  A.ax += bx;
-  A.ay += by;
+  RefRates A = ref_finish(P, o, sums, bx, by);
   if (P.gravity_flag == 1) {
     A.ay -= P.g;
     A.ay_a -= P.g;
@@ -299,11 +347,10 @@ __device__ __forceinline__ void ref_epilogue(const DevParams &P, const SlotArray
 // same in both buffers and are not written.  S is only read here, at the
 // particle's own slot.
 __device__ __forceinline__ void ref_step_epilogue(const DevParams &P, const SlotArrays &S, const StepOut &F, int a,
-                                                  const RefOwn &o, RefAcc &A, double bx, double by)
+                                                  const RefOwn &o, const RefAcc &sums, double bx, double by)
 {
   const SlotArrays &D = F.D;
-  A.ax += bx;
-  A.ay += by;
+  RefRates A = ref_finish(P, o, sums, bx, by);
   if (P.gravity_flag == 1) {
     A.ay -= P.g;
     A.ay_a -= P.g;
@@ -403,7 +450,7 @@ struct GlobalSrc {
   __device__ __forceinline__ float2 xyf(int) const { return make_float2(0.f, 0.f); }  // not used: no pre-test
   __device__ __forceinline__ int orig(int s) const { return S.orig[s]; }
   __device__ __forceinline__ double mass(int s) const { return S.m[s]; }
-  __device__ __forceinline__ RefRec get(int s) const { return load_ref_rec(P, S, s); }
+  __device__ __forceinline__ RefRec get(int s) const { return load_ref_rec(S, s); }
   __device__ __forceinline__ void cut(int s, double &d2, int &j) const
   {
     d2 = P.kcut_d2[s];
@@ -411,36 +458,24 @@ struct GlobalSrc {
   }
 };
 // Phase 1 and 2 for one own particle until its stencil is exhausted.
-// nshort >= 0: the own particle's candidate list, nshort entries, is in its
-// column of s_nb (kF32 only); else the stencil is walked, appending to
-// vl_out (if not null) as tile_list does.
 template <bool kBrute, bool kKnn, bool kF32, typename Src, typename Cursor, typename Entry>
 __device__ __forceinline__ void ref_particle(const DevParams &P, const Src &src, Cursor &cur, bool active, int self,
                                              const RefOwn &o, const F32Test &ft, Entry *s_nb, RefAcc &A, double &bx,
-                                             double &by, unsigned &my_pairs, int &my_nb, double cd, int cj,
-                                             int nshort, unsigned short *vl_out, int &vl_cnt)
+                                             double &by, unsigned &my_pairs, int &my_nb, double cd, int cj)
 {
   constexpr Entry kRole = sizeof(Entry) == 2 ? (Entry)kRoleI16 : (Entry)kRoleI;
   const int col = threadIdx.x;
   bool more = active;
   while (__any_sync(0xffffffffu, more)) {
-    int cnt = 0;
-    if (kF32 && nshort >= 0) {
-      if constexpr (kF32) {
-        if (more)
-          cnt = tile_list_short<kBrute, kKnn>(P, src, nshort, self, o.r.orig, o.r.x, o.r.y, ft, s_nb, col, my_pairs,
-                                              my_nb, bx, by, cd, cj);
-      }
-      more = false;
-    } else {
-      cnt = tile_list<kBrute, kTileChunk, kKnn, kF32>(P, src, cur, more, self, o.r.orig, o.r.x, o.r.y, ft, s_nb, col,
-                                                      my_pairs, my_nb, bx, by, cd, cj, vl_out, vl_cnt);
-    }
+    const int cnt = tile_list<kBrute, kTileChunk, kKnn, kF32>(P, src, cur, more, self, o.r.orig, o.r.x, o.r.y, ft, s_nb,
+                                                              col, my_pairs, my_nb, bx, by, cd, cj);
     __syncwarp();
     for (int e = 0; e < cnt; e++) {
       const Entry ent = s_nb[e * kTileThreads + col];
       const RefRec b = src.get((int)(ent & (Entry)~kRole));
-      ref_pair(P, o, b, (ent & kRole) != 0, A);
+      const double dxa = o.r.x - b.x, dya = o.r.y - b.y;
+      const bool isI = (ent & kRole) != 0;
+      ref_pair<false>(P, o, b, dxa, dya, exact_r2(dxa, dya), isI, true, isI && o.r.itype == 1 && b.itype >= 2, A);
     }
     __syncwarp();
   }
@@ -449,7 +484,7 @@ __device__ __forceinline__ void ref_particle(const DevParams &P, const Src &src,
 // Dynamic shared memory of the tiled pass and its record capacity; with the
 // knn cap every record also carries its query's cut (12 bytes).
 template <bool kKnn>
-__host__ __device__ constexpr int ref_rec_cap() { return kKnn ? 560 : 620; }
+__host__ __device__ constexpr int ref_rec_cap() { return kKnn ? 720 : 800; }
 constexpr size_t kRefListBytes = sizeof(unsigned short) * kTileChunk * kTileThreads;
 // per record: the record, its FP32 position and (kKnn) its cut
 template <bool kKnn>
@@ -457,7 +492,7 @@ constexpr size_t ref_smem()
 {
   return sizeof(TileBlock) + kRefListBytes + (sizeof(RefRec) + 8 + (kKnn ? 12 : 0)) * ref_rec_cap<kKnn>();
 }
-static_assert(sizeof(RefRec) * 560 >= sizeof(unsigned) * kTileChunk * kTileThreads,
+static_assert(sizeof(RefRec) * 720 >= sizeof(unsigned) * kTileChunk * kTileThreads,
               "the fallback's 32-bit lists live in the record area");
 
 // One CTA per storage tile (see tile_pass.cuh).  Phase 1 lists in-radius
@@ -491,10 +526,6 @@ __device__ __forceinline__ void ref_tile(const DevParams &P, const SlotArrays &S
   // the origin of the block: the listing's FP32 positions are relative to it
   const double ox = P.lo_x + B.bx0 * P.cell, oy = P.lo_y + B.by0 * P.cell;
   if (staged) {
-    // this tile's candidate lists are current if written since the last
-    // build (G.vl null: the lists are off, every particle walks the stencil)
-    const unsigned gen = G.vl ? *G.gen : 0u;
-    const bool vl_use = G.vl && G.tile_gen[tile] == gen;
     // two records per thread at a time, every load issued before the first
     // store, so the staging waits for two rounds of loads (the slots, then
     // their fields) instead of two per record
@@ -511,20 +542,8 @@ __device__ __forceinline__ void ref_tile(const DevParams &P, const SlotArrays &S
       const bool two = k1 < B.nrec;
       const int s0 = G.list[tile_record_pos(B, k0)];
       const int s1 = two ? G.list[tile_record_pos(B, k1)] : s0;
-      // the candidate lists the core's fluid particles will read after the
-      // staging: fetched into L2 meanwhile (the halo's too, for their tiles)
-      if (vl_use) {
-        if (s0 < P.nf) {
-          prefetch_l2(G.vl + (size_t)s0 * kVlMax);
-          prefetch_l2(G.vl_n + s0);
-        }
-        if (two && s1 < P.nf) {
-          prefetch_l2(G.vl + (size_t)s1 * kVlMax);
-          prefetch_l2(G.vl_n + s1);
-        }
-      }
-      const RefRec r0 = load_ref_rec(P, S, s0);
-      const RefRec r1 = load_ref_rec(P, S, s1);
+      const RefRec r0 = load_ref_rec(S, s0);
+      const RefRec r1 = load_ref_rec(S, s1);
       // only fluid queries have a cut; other records are never a pair's i
       // seen from a fluid particle that is its j
       double cd0 = 0.0, cd1 = 0.0;
@@ -570,16 +589,11 @@ __device__ __forceinline__ void ref_tile(const DevParams &P, const SlotArrays &S
       int cj = 0;
       if (kKnn && active) src.cut(kr, cd, cj);
       const float2 of = s_posf[active ? kr : 0];
-      const F32Test ft = make_f32_test(P, B, of.x, of.y);
-      int nshort = -1, vl_cnt = 0;
-      unsigned short *vl_out = nullptr;
-      if (active && G.vl) nshort = load_candidates(G, a, vl_use, s_nb16, threadIdx.x, vl_out);
+      const F32Test ft = make_f32_test(P, max(B.W, B.H), of.x, of.y);
       RefAcc A = {};
       double bx = 0.0, by = 0.0;
       int nb = 0;
-      ref_particle<kBrute, kKnn, true>(P, src, cur, active, kr, o, ft, s_nb16, A, bx, by, my_pairs, nb, cd, cj, nshort,
-                                       vl_out, vl_cnt);
-      if (vl_out) G.vl_n[a] = vl_cnt <= kVlMax ? (unsigned char)vl_cnt : kVlOverflow;
+      ref_particle<kBrute, kKnn, true>(P, src, cur, active, kr, o, ft, s_nb16, A, bx, by, my_pairs, nb, cd, cj);
       my_nb = max(my_nb, nb);
       if (active) {
         if (F.enabled)
@@ -588,7 +602,6 @@ __device__ __forceinline__ void ref_tile(const DevParams &P, const SlotArrays &S
           ref_epilogue(P, S, a, o, A, bx, by);
       }
     }
-    if (G.vl && !vl_use && threadIdx.x == 0) G.tile_gen[tile] = gen;
   } else {
     // a crowded tile: the same walk over the cell list in global memory
     unsigned *s_nb32 = reinterpret_cast<unsigned *>(rec);
@@ -602,7 +615,7 @@ __device__ __forceinline__ void ref_tile(const DevParams &P, const SlotArrays &S
       }
       const bool active = k < ncore && a < P.nf;
       const int as = active ? a : 0;
-      const RefOwn o = make_own(P, load_ref_rec(P, S, as));
+      const RefOwn o = make_own(P, load_ref_rec(S, as));
       GlobalCursor cur;
       cur.list = G.list;
       cur.c.init(P, G, G.cell_of[as]);
@@ -613,9 +626,7 @@ __device__ __forceinline__ void ref_tile(const DevParams &P, const SlotArrays &S
       RefAcc A = {};
       double bx = 0.0, by = 0.0;
       int nb = 0;
-      int vl_none = 0;
-      ref_particle<kBrute, kKnn, false>(P, src, cur, active, as, o, ft, s_nb32, A, bx, by, my_pairs, nb, cd, cj, -1,
-                                        nullptr, vl_none);
+      ref_particle<kBrute, kKnn, false>(P, src, cur, active, as, o, ft, s_nb32, A, bx, by, my_pairs, nb, cd, cj);
       my_nb = max(my_nb, nb);
       if (active) {
         if (F.enabled)
@@ -675,6 +686,109 @@ uph_status launch_ref_pass(const DevParams &P, const SlotArrays &S, const CellGr
   if (P.knn > 0)
     return brute ? launch_ref<true, true>(P, S, G, st, F, s) : launch_ref<false, true>(P, S, G, st, F, s);
   return brute ? launch_ref<true, false>(P, S, G, st, F, s) : launch_ref<false, false>(P, S, G, st, F, s);
+}
+
+// ---- a step in one launch (tile_stream.cuh) -------------------------------------------
+template <bool kBrute>
+struct RefStream {
+  static constexpr int kStride = sizeof(RefRec);
+  const DevParams &P;
+  const SlotArrays &S;
+  const StepOut &F;
+  unsigned my_pairs;
+  int my_nb;
+
+  __device__ __forceinline__ void stage(int s, uint32_t dst) const
+  {
+    const double *f[13] = {S.x, S.y, S.u, S.v, S.ut, S.vt, S.rho, S.rhot, S.p, S.pt, S.m, S.inv_rhot, S.inv_rho};
+#pragma unroll
+    for (int k = 0; k < 13; k++) cp_async8(dst + 8 * k, f[k] + s);
+    cp_async4(dst + 108, S.itype + s);
+  }
+  __device__ __forceinline__ void convert(int, unsigned char *, unsigned char *) const {}
+  // the epilogue's reads of the particle's own *_min state and sponge
+  // factor: fetched into L2 while the tile arrives and its pairs are summed
+  __device__ __forceinline__ void begin(int a) const
+  {
+    if (!F.enabled || a < 0) return;
+    if (!F.first_step || !F.predict_next) {
+      prefetch_l2(S.rho_min + a);
+      prefetch_l2(S.p_min + a);
+      prefetch_l2(S.u_min + a);
+      prefetch_l2(S.v_min + a);
+    }
+    if (P.moving_boundary == 1 && P.wave_absorption == 1) prefetch_l2(S.sponge + a);
+  }
+  template <int kLanes, typename Stream>
+  __device__ __forceinline__ void particle(const unsigned char *buf, int rec, int a, int n, CandReader<kLanes> &rd,
+                                           Stream &stream)
+  {
+    const RefRec *r = reinterpret_cast<const RefRec *>(buf);
+    const RefOwn o = make_own(P, r[rec]);
+    RefAcc A = {};
+    double bx = 0.0, by = 0.0;
+    int nb = 0;
+    const int most = max(__reduce_max_sync(0xffffffffu, n), Stream::kReadyAt + 1);
+    for (int e = 0; e < most; e++) {
+      stream.refill(e);
+      const unsigned c = rd.next(e);
+      const RefRec b = r[e < n ? (int)(c & kCandRec) : rec];
+      const double dxa = o.r.x - b.x, dya = o.r.y - b.y;
+      const double r2 = exact_r2(dxa, dya);
+      // r^2 is not negative: its bits order like its value (and a NaN, in
+      // either sign, is above every bound)
+      const unsigned long long bits = __double_as_longlong(r2);
+      const bool in = e < n && bits < __double_as_longlong(P.r2cut);
+      if (kBrute && in && (c & kCandBoundary)) brute_wall_force(P, r2, dxa, dya, b.m, bx, by);
+      const bool near = in && bits > __double_as_longlong(DBL_EPSILON);
+      nb += near;
+      const bool on = near && !(c & kCandNoPair);
+      const bool isI = (c & kCandI) != 0u;
+      my_pairs += on && isI;
+      ref_pair<true>(P, o, b, dxa, dya, r2, isI, on, on && (c & kCandWall), A);
+    }
+    stream.done_reading();
+    if constexpr (kLanes > 1) {
+      double *sums = reinterpret_cast<double *>(&A);
+#pragma unroll
+      for (int k = 0; k < (int)(sizeof(RefAcc) / sizeof(double)); k++) sums[k] = lanes_sum<kLanes>(sums[k]);
+      bx = lanes_sum<kLanes>(bx);
+      by = lanes_sum<kLanes>(by);
+      nb = lanes_sum<kLanes>(nb);
+    }
+    my_nb = max(my_nb, nb);
+    if (a < 0 || (threadIdx.x & (kLanes - 1)) != 0) return;
+    if (F.enabled)
+      ref_step_epilogue(P, S, F, a, o, A, bx, by);
+    else
+      ref_epilogue(P, S, a, o, A, bx, by);
+  }
+};
+
+template <bool kBrute, int kLanes>
+__global__ void __launch_bounds__(kTileThreads, 2) k_ref_step(const CellBuildArgs C, const SlotArrays S, const StepOut F,
+                                                           const StepArgs A)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  RefStream<kBrute> ps{C.P, S, F, 0u, 0};
+  step_run<kBrute, kLanes>(C, S, F, A, ps, smem, [&](int tile) {
+    ref_tile<kBrute, false>(C.P, S, C.G, F, tile, smem, ps.my_pairs, ps.my_nb);
+  });
+}
+
+uph_status launch_ref_step(const DevParams &P, const SlotArrays &S, const CellGrid &G, const StepOut &F,
+                           const StepArgs &A, unsigned *err, cudaStream_t s)
+{
+  const bool brute = P.boundary_force != 3 && P.boundary_force != 4 && P.boundary_force != 5;
+  constexpr size_t sm = std::max({ref_smem<false>(), stream_smem_bytes<sizeof(RefRec)>(), kRecordSmemBytes});
+  if (P.lanes == 4)
+    return brute ? launch_step<k_ref_step<true, 4>>(sm, P, S, G, F, A, err, s)
+                 : launch_step<k_ref_step<false, 4>>(sm, P, S, G, F, A, err, s);
+  if (P.lanes == 2)
+    return brute ? launch_step<k_ref_step<true, 2>>(sm, P, S, G, F, A, err, s)
+                 : launch_step<k_ref_step<false, 2>>(sm, P, S, G, F, A, err, s);
+  return brute ? launch_step<k_ref_step<true, 1>>(sm, P, S, G, F, A, err, s)
+               : launch_step<k_ref_step<false, 1>>(sm, P, S, G, F, A, err, s);
 }
 
 // The knn cap's cut of every fluid query: walk the stencil (the global cell
@@ -909,7 +1023,7 @@ __global__ void __launch_bounds__(128) k_packing_pass(const DevParams P, const S
     const int ita = S.itype[a];
     const double cd = kKnn ? P.kcut_d2[a] : 0.0;
     const int cj = kKnn ? P.kcut_j[a] : 0;
-    RefAcc A = {};
+    RefRates A = {};
     double gx = 0.0, gy = 0.0, bx = 0.0, by = 0.0;
     int np = 0;
     NeighbourCursor cur;
@@ -935,7 +1049,7 @@ __global__ void __launch_bounds__(128) k_packing_pass(const DevParams P, const S
       gx = fma(F, dx, gx);
       gy = fma(F, dy, gy);
       np++;
-      if (isI && ita == 1 && S.itype[b] >= 2) wall_pair_force(P, S.itype[b], r2, dx, dy, ua - S.u[b], va - S.v[b], ma, A);
+      if (isI && ita == 1 && S.itype[b] >= 2) wall_pair_force(P, S.itype[b], r2, dx, dy, ua - S.u[b], va - S.v[b], ma, A.ax, A.ay, A.ax_a, A.ay_a);
     }
     const double V0 = *P.pack_mass0 / P.rho0;
     const double beta = 2.0 * P.g * P.local_depth;

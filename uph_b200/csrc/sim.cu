@@ -19,7 +19,7 @@
 #include <string>
 #include <vector>
 
-#include "tile_pass.cuh"
+#include "tile_stream.cuh"
 #include "sim_access.cuh"
 
 using namespace uph;
@@ -77,9 +77,11 @@ struct uph_sim {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   unsigned *d_err = nullptr;
-  // the rate pass's statistics, zeroed by the cell-list launch before it
+  // the rate pass's statistics, zeroed by the cell-list launch before it or
+  // published by the step's launch, and that launch's running sums
   unsigned long long *d_niac = nullptr;
   int *d_max_nb = nullptr;
+  unsigned *d_step_done = nullptr, *d_moved = nullptr, *d_phases = nullptr;
   int *d_perm = nullptr;  // scratch for uploads
   int itime = 0;
   int steps_since_reorder = 0;
@@ -112,7 +114,7 @@ struct uph_sim {
   // tuning: storage re-sort interval and the grid arrays' capacity in cells
   int reorder_interval = kReorderInterval;
   long long grid_capacity = 0;
-  long long tile_gen_capacity = 0;
+  long long stream_tiles = 0;  // storage tiles the stream's per-tile arrays hold
   // the fluid state was replaced from outside (the learned surrogate): the
   // next step starts the leapfrog afresh with the first-step half kick
   bool restart = false;
@@ -433,8 +435,21 @@ uph_status check_error_word(uph_sim *s)
     cudaMemsetAsync(s->G.count, 0, sizeof(int) * s->G.ncell, s->stream);
     cudaMemsetAsync(s->G.bar, 0, kGridWords * sizeof(unsigned), s->stream);
     cudaMemsetAsync(s->d_err, 0, sizeof(unsigned), s->stream);
+    cudaMemsetAsync(s->d_phases, 0, 2 * TicketPhases::kPhases * sizeof(unsigned), s->stream);
+    cudaMemsetAsync(s->P.rebuild, 1, sizeof(unsigned), s->stream);  // and the list is built afresh
     return fail(UPH_TIMEOUT, "a device-side wait timed out");
   }
+  return UPH_OK;
+}
+
+// what follows the rate pass of an evaluation
+uph_status after_pass(uph_sim *s)
+{
+  if (s->P.stress_type == 2 && s->P.profile == UPH_PROFILE_REF && s->P.flag_init_simul == 1) {
+    launch_viscous_two_step(s->P, s->S, s->G, s->stream);
+    s->launches += 2;
+  }
+  s->have_rates = true;
   return UPH_OK;
 }
 
@@ -452,7 +467,27 @@ uph_status rate_pass(uph_sim *s, bool refresh, bool step = false, const StepOut 
     s->launches++;
   }
   const PassStats st{s->d_niac, s->d_max_nb};
-  uph_status r = build_cell_list(s, &st, step ? s->d_itime : nullptr);
+  uph_status r;
+  // the steps of uph_sim_step: one launch, the cell list in it (a lone
+  // evaluation, after an upload that rebuilt the list, would only write
+  // candidate lists nobody reads)
+  if (step && s->P.knn == 0 && s->P.nf > 0 &&
+      (s->P.profile != UPH_PROFILE_REF || s->P.flag_init_simul == 1)) {
+    Timer t(s, KF_PASS);
+    const StepArgs A{PassStats{s->d_niac + 1, s->d_max_nb + 1}, st, s->d_step_done, s->d_moved, s->d_step_done + 4, s->d_phases,
+                     s->cand_lists ? 0 : 1, s->d_itime};
+    const StepOut out = F ? *F : StepOut{};
+    r = s->P.profile != UPH_PROFILE_REF ? launch_wcsph_step(s->P, s->S, s->G, out, A, s->d_err, s->stream)
+                                        : launch_ref_step(s->P, s->S, s->G, out, A, s->d_err, s->stream);
+    if (r != UPH_OK) return r;
+    s->launches++;
+    if (s->P.nvrules > 0) {
+      launch_virtual(s->P, s->S, s->vb, s->deriv_t, s->d_itime, s->stream);
+      s->launches += 3;
+    }
+    return after_pass(s);
+  }
+  r = build_cell_list(s, &st, step ? s->d_itime : nullptr);
   if (r != UPH_OK) return r;
   VirtualPoints vp = {nullptr, nullptr, CellGrid{}};
   if (s->P.nvrules > 0) {
@@ -473,28 +508,15 @@ uph_status rate_pass(uph_sim *s, bool refresh, bool step = false, const StepOut 
     s->kcut_fresh = true;
   }
   Timer t(s, KF_PASS);
-  // the tiled passes' candidate lists (uph_sim_set_candidate_lists), for
-  // the steps of uph_sim_step: a lone evaluation (uph_sim_derivatives, after
-  // an upload that rebuilt the list) would only write lists nobody reads
-  CellGrid gp = s->G;
-  if (!s->cand_lists || !step) {
-    gp.vl = nullptr;
-    gp.vl_n = nullptr;
-  }
   if (s->P.profile != UPH_PROFILE_REF)
-    r = launch_wcsph_pass(s->P, s->S, gp, st, F ? *F : StepOut{}, s->stream);
+    r = launch_wcsph_pass(s->P, s->S, s->G, st, F ? *F : StepOut{}, s->stream);
   else if (s->P.flag_init_simul == 0)
     r = launch_packing_pass(s->P, s->S, s->G, st, s->stream);
   else
-    r = launch_ref_pass(s->P, s->S, gp, st, F ? *F : StepOut{}, s->stream);
+    r = launch_ref_pass(s->P, s->S, s->G, st, F ? *F : StepOut{}, s->stream);
   if (r != UPH_OK) return r;
   s->launches++;
-  if (s->P.stress_type == 2 && s->P.profile == UPH_PROFILE_REF && s->P.flag_init_simul == 1) {
-    launch_viscous_two_step(s->P, s->S, s->G, s->stream);
-    s->launches += 2;
-  }
-  s->have_rates = true;
-  return UPH_OK;
+  return after_pass(s);
 }
 
 uph_status validate(const uph_params *p)
@@ -539,18 +561,27 @@ cudaError_t alloc_grid(uph_sim *s)
   G.ncell = (int)ncell;
   G.nblock_sums = scan_block_sums_needed((int)ncell);
   s->gv.ncell = (int)ncell;
-  // the tiles' candidate-list generations: none matches any build's
+  // the recorded tiles of the passes that stream (tile_stream.cuh): a
+  // recorded tile holds a fluid particle, and a tile of the default edge
+  // about 225 of them; one beyond the capacity is handled as a hard tile
   const long long ntiles = (long long)s->P.ntx * (s->P.ncy / s->P.tile);
-  if (ntiles > s->tile_gen_capacity) {
-    if (G.tile_gen) cudaFree(G.tile_gen);
-    G.tile_gen = nullptr;
-    cudaError_t e = cudaMalloc((void **)&G.tile_gen, sizeof(unsigned) * ntiles);
-    if (e != cudaSuccess) return e;
-    s->tile_gen_capacity = ntiles;
-  }
-  if (ntiles > 0) {
-    cudaError_t e = cudaMemset(G.tile_gen, 0xff, sizeof(unsigned) * ntiles);
-    if (e != cudaSuccess) return e;
+  const long long want = std::min(ntiles, (long long)s->P.nf / 64 + 1024);
+  if (ntiles > s->stream_tiles) {
+    StreamTiles &t = G.st;
+    for (void *p : {(void *)t.slot, (void *)t.core, (void *)t.tile, (void *)t.hard, (void *)t.live})
+      if (p) cudaFree(p);
+    t.slot = t.tile = t.hard = t.live = nullptr;
+    t.core = nullptr;
+    t.cap = 0;
+    s->stream_tiles = 0;
+    cudaError_t e;
+    if ((e = cudaMalloc((void **)&t.slot, sizeof(int) * want * kStreamCap)) != cudaSuccess) return e;
+    if ((e = cudaMalloc((void **)&t.core, sizeof(int2) * want * kTileThreads)) != cudaSuccess) return e;
+    if ((e = cudaMalloc((void **)&t.tile, sizeof(int) * want)) != cudaSuccess) return e;
+    if ((e = cudaMalloc((void **)&t.hard, sizeof(int) * ntiles)) != cudaSuccess) return e;
+    if ((e = cudaMalloc((void **)&t.live, sizeof(int) * ntiles)) != cudaSuccess) return e;
+    t.cap = (int)want;
+    s->stream_tiles = ntiles;
   }
   // cudaMemset runs on the legacy default stream, which the simulation's
   // non-blocking stream does not wait for: the memsets here must have
@@ -586,6 +617,15 @@ cudaError_t alloc_grid(uph_sim *s)
 // adds candidates -- the pair test is the exact distance predicate.
 constexpr double kMaxGridCells = double(1 << 26);
 
+// Up to these many fluid particles a step's pass runs on smaller tiles with
+// four or two lanes per particle (tile_stream.cuh).  us per step of a
+// stirred dam break, REF: tile 5 x 4 lanes / tile 7 x 2 / tile 11 x 1:
+// 3,000 particles 17.9 / 19.9 / 29.4; 14,000 25.9 / 26.1 / 30.6; 20,000
+// 27.4 / 24.8 / 30.5; 28,000 33.0 / 32.0 / 34.4; 40,000 41.6 / 37.4 / 38.5
+// (WCSPH FP64 28,000 34.1 / 33.5 / 33.5; 40,000 41.6 / 37.3 / 34.4).  FP32 pairs stay with
+// one lane: their sums are FP32 and keep their order.
+constexpr int kFourLanesMax = 15000, kTwoLanesMax = 30000;
+
 void set_grid_geometry(DevParams &P, int reach, int tile)
 {
   P.reach = reach;
@@ -608,6 +648,13 @@ void set_grid_geometry(DevParams &P, int reach, int tile)
   P.ntx = (int)tiles_x;
   P.ncx = P.ntx * tile;
   P.ncy = (int)tiles_y * tile;
+  // lanes per particle of a step's pass: as many as a tile's core particles
+  // (with a tenth to spare for compression) leave of a CTA's threads, where
+  // the tiles do not fill the machine anyway
+  const double core = P.dx > 0 ? 1.1 * (tile * cell / P.dx) * (tile * cell / P.dx) : 1e9;
+  P.lanes = 1;
+  if (P.nf <= kTwoLanesMax && P.precision != UPH_PREC_FP32_PAIR)
+    P.lanes = core * 4 <= kTileThreads ? 4 : core * 2 <= kTileThreads ? 2 : 1;
 }
 
 // The mirror rules of each virtualType, in the reference's loop order
@@ -700,6 +747,7 @@ DevParams make_dev_params(const uph_params *p)
   P.gravity_flag = p->gravity_flag;
   P.mu0 = p->viscosity0;
   P.two_mu0 = 2.0 * p->viscosity0;
+  P.gamma4 = 4.0 * p->adiabatic_constant;
   P.kappa = p->thermal_diffusivity0;
   P.eps = p->epsilon;
   P.stress_type = p->stress_type;
@@ -743,6 +791,8 @@ DevParams make_dev_params(const uph_params *p)
   int tile = kCellTile;
   const double hdx = p->dx > 0 ? h / p->dx : 1.0;
   if (hdx > 1.4) tile = std::max(2, (int)floor(kCellTile * 1.3 / hdx));
+  if (p->n_fluid <= kTwoLanesMax && p->precision != UPH_PREC_FP32_PAIR && p->knn_cap == 0)
+    tile = std::max(2, tile * (p->n_fluid <= kFourLanesMax ? 5 : 7) / kCellTile);
   set_grid_geometry(P, kCellReach, tile);
   P.knn = p->knn_cap;
   P.kcut_d2 = nullptr;
@@ -809,7 +859,28 @@ extern "C" uph_status uph_sim_create(const uph_params *p, uph_sim **out)
   TRY(cudaMemset(s->P.rebuild, 1, sizeof(unsigned)));
   TRY(dalloc(s, &G.gen, 1));
   TRY(cudaMemset(G.gen, 0, sizeof(unsigned)));
-  TRY(dalloc(s, &G.vl, (size_t)nf * kVlMax));
+  {
+    // room for 1.3 times the candidates of a lattice (pi (R_l / dx)^2, R_l
+    // the list radius), so that moving water seldom overflows: 32 entries at
+    // h = 1.3 dx
+    const double Rl = sqrt(s->P.r2cut) + 2.0 * 1.4142135623730951 * s->P.skin;
+    const double want = 1.3 * 3.14159 * (Rl / p->dx) * (Rl / p->dx);
+    G.vl_cap = want >= kVlCapMax ? kVlCapMax : std::max(16, (int)ceil(want / 8.0) * 8);
+  }
+  TRY(dalloc(s, &G.vl, (size_t)nf * G.vl_cap));
+  {
+    int *w = nullptr;  // nstream, nhard, recorded, nlive; the step's finished blocks, skin flag, tile ticket and build phases
+    constexpr int kWords = 8 + 2 * TicketPhases::kPhases;
+    TRY(dalloc(s, &w, kWords));
+    TRY(cudaMemset(w, 0, kWords * sizeof(int)));
+    G.st.nstream = w;
+    G.st.nhard = w + 1;
+    G.st.recorded = reinterpret_cast<unsigned *>(w + 2);
+    s->d_step_done = reinterpret_cast<unsigned *>(w + 3);
+    s->d_moved = reinterpret_cast<unsigned *>(w + 4);
+    G.st.nlive = w + 5;
+    s->d_phases = reinterpret_cast<unsigned *>(w + 8);
+  }
   TRY(dalloc(s, &G.vl_n, (size_t)nf));
   TRY(dalloc(s, &G.rank, (size_t)n));
   TRY(dalloc(s, &G.totals, (size_t)kCellBuildMaxBlocks + 1));
@@ -847,8 +918,10 @@ extern "C" uph_status uph_sim_create(const uph_params *p, uph_sim **out)
   double **tfl2[] = {&T.vmin, &T.acc, &T.acc_a, &T.fvel};
   for (double **q : tfl2) TRY(dalloc(s, q, 2 * (size_t)nf));
   TRY(dalloc(s, &s->d_err, 1));
-  TRY(dalloc(s, &s->d_niac, 1));
-  TRY(dalloc(s, &s->d_max_nb, 1));
+  TRY(dalloc(s, &s->d_niac, 2));  // the last pass's; a step's running sums
+  TRY(dalloc(s, &s->d_max_nb, 2));
+  TRY(cudaMemset(s->d_niac, 0, 2 * sizeof(unsigned long long)));
+  TRY(cudaMemset(s->d_max_nb, 0, 2 * sizeof(int)));
   TRY(dalloc(s, &s->d_perm, (size_t)n));
   TRY(dalloc(s, &s->d_itime, 1));
   TRY(dalloc(s, &s->d_wall_tab, 4 * (size_t)(p->n_moving > 0 ? p->n_moving : 1)));
@@ -893,7 +966,8 @@ extern "C" uph_status uph_sim_destroy(uph_sim *s)
   drop_graph(s);
   for (void *p : s->allocations) cudaFree(p);
   for (void *p : {(void *)s->G.count, (void *)s->G.start, (void *)s->G.fill, (void *)s->G.block_sums,
-                  (void *)s->G.tile_gen,
+                  (void *)s->G.st.slot, (void *)s->G.st.core, (void *)s->G.st.tile, (void *)s->G.st.hard,
+                  (void *)s->G.st.live,
                   (void *)s->gv.count, (void *)s->gv.start, (void *)s->gv.fill, (void *)s->pe_ip, (void *)s->pe_jp,
                   (void *)s->pe_r2, (void *)s->pe_w, (void *)s->pe_dw})
     if (p) cudaFree(p);

@@ -220,10 +220,11 @@ struct F32Test {
   float vl;      // the candidate lists' radius squared (1 + band)
 };
 
-__device__ __forceinline__ F32Test make_f32_test(const DevParams &P, const TileBlock &B, float xa, float ya)
+// cells: the block's larger edge in cells
+__device__ __forceinline__ F32Test make_f32_test(const DevParams &P, int cells, float xa, float ya)
 {
   const double R = sqrt(P.r2cut);
-  const double E = (double)max(B.W, B.H) * P.cell;
+  const double E = (double)cells * P.cell;
   const double band = 32.0 * (E / R) * 0x1p-23 + 0x1p-20;
   // between two builds a particle moves at most the skin along each axis,
   // so a pair's distance shrinks by at most 2 sqrt(2) skin
@@ -232,43 +233,119 @@ __device__ __forceinline__ F32Test make_f32_test(const DevParams &P, const TileB
                  (float)(P.r2cut * 1e-3), (float)(Rl * Rl * (1.0 + band))};
 }
 
-// The own particle's (slot a) candidate list for its listing.  use (the
-// tile's lists are current) and no overflow: the entries are copied into
-// column col of s_nb and their count returned.  Else -1: the stencil is
-// walked, and vl_out points at the particle's list to write meanwhile (null
-// when the lists are current but this one overflowed).
-static_assert(kVlMax == 24 && kVlMax <= kTileChunk, "a candidate list is three 16-byte words and fits a column");
-__device__ __forceinline__ int load_candidates(const CellGrid &G, int a, bool use, unsigned short *s_nb, int col,
-                                               unsigned short *&vl_out)
+// ---- candidate lists (tile_stream.cuh) ------------------------------------------------
+// An entry: the record's index in its block and the pair's roles, which are
+// constants of the particles.
+constexpr unsigned kCandRec = 0x1ffu;
+constexpr unsigned kCandI = 0x200u;         // the own particle is the pair's i
+constexpr unsigned kCandNoPair = 0x400u;    // within ParticleBoundary's exclusion: counted, never a pair
+constexpr unsigned kCandWall = 0x800u;      // a listed pair's wall force acts (i side fluid, partner a wall)
+constexpr unsigned kCandBoundary = 0x1000u; // a boundary particle (the brute-force wall modes)
+static_assert(kStreamCap <= (int)kCandRec + 1, "a record index fits its bits");
+
+// A particle's list in CellGrid::vl: entry e of slot a is at
+// vl[((e / 8) nf + a) 8 + e % 8], so that a warp's 16-byte words of eight
+// entries lie side by side.
+// Reads a list in order: lane l of a particle's kLanes lanes takes the
+// entries l, l + kLanes, ...
+template <int kLanes>
+struct CandReader;
+// one lane: eight entries (one 16-byte word) at a time, the next word
+// fetched while the current one is used
+template <>
+struct CandReader<1> {
+  const uint4 *p;
+  size_t stride;
+  uint4 w, nx;
+  int n;
+
+  // slot a's list (a < 0: an empty one); returns its length.  The first two
+  // words are fetched beside the length (vl_cap is at least 16).
+  __device__ __forceinline__ int init(const CellGrid &G, int nf, int a)
+  {
+    p = reinterpret_cast<const uint4 *>(G.vl) + max(a, 0);
+    stride = (size_t)nf;
+    n = 0;
+    w = nx = make_uint4(0u, 0u, 0u, 0u);
+    if (a >= 0) {
+      n = G.vl_n[a];
+      w = p[0];
+      nx = p[stride];
+    }
+    p += stride;
+    return n;
+  }
+  // entry e of the list (e = 0, 1, ... in turn)
+  __device__ __forceinline__ unsigned next(int e)
+  {
+    if (e != 0 && (e & 7) == 0) {
+      w = nx;
+      p += stride;
+      if (e + 8 < n) nx = *p;
+    }
+    const unsigned k = w.x & 0xffffu;
+    w.x = __funnelshift_r(w.x, w.y, 16);
+    w.y = __funnelshift_r(w.y, w.z, 16);
+    w.z = __funnelshift_r(w.z, w.w, 16);
+    w.w >>= 16;
+    return k;
+  }
+};
+// several lanes: an entry at a time, the next one fetched a turn ahead
+template <int kLanes>
+struct CandReader {
+  const unsigned short *p;
+  size_t stride;
+  unsigned nx;
+  int n, lane;  // the particle's list, this lane's part of it
+
+  __device__ __forceinline__ unsigned fetch(int e) const
+  {
+    const int k = e * kLanes + lane;
+    return p[(size_t)(k >> 3) * stride + (k & 7)];
+  }
+  // returns how many entries this lane takes
+  __device__ __forceinline__ int init(const CellGrid &G, int nf, int a)
+  {
+    lane = threadIdx.x & (kLanes - 1);
+    p = G.vl + 8 * (size_t)max(a, 0);
+    stride = 8 * (size_t)nf;
+    nx = 0;
+    if (a < 0) return n = 0;
+    n = G.vl_n[a];
+    nx = fetch(0);
+    return n = (n - lane + kLanes - 1) / kLanes;
+  }
+  __device__ __forceinline__ unsigned next(int e)
+  {
+    const unsigned k = nx;
+    if (e + 1 < n) nx = fetch(e + 1);
+    return k;
+  }
+};
+// a sum over a particle's lanes, the same in each of them
+template <int kLanes>
+__device__ __forceinline__ double lanes_sum(double v)
 {
-  vl_out = nullptr;
-  if (!use) {
-    vl_out = G.vl + (size_t)a * kVlMax;
-    return -1;
-  }
-  const uint4 *w = reinterpret_cast<const uint4 *>(G.vl + (size_t)a * kVlMax);
-  const uint4 w0 = w[0], w1 = w[1], w2 = w[2];
-  const int n = G.vl_n[a];
-  if (n == kVlOverflow) return -1;
-  const unsigned v[12] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
 #pragma unroll
-  for (int q = 0; q < 12; q++) {
-    if (2 * q < n) s_nb[(2 * q) * kTileThreads + col] = (unsigned short)(v[q] & 0xffffu);
-    if (2 * q + 1 < n) s_nb[(2 * q + 1) * kTileThreads + col] = (unsigned short)(v[q] >> 16);
-  }
-  return n;
+  for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <int kLanes>
+__device__ __forceinline__ int lanes_sum(int v)
+{
+#pragma unroll
+  for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
 // One batch of kB candidates b[] (the own index `self` for none) of the
 // listing: the FP32 pre-test (kF32), the exact predicate and the pair
 // filters; each listed partner goes to row cnt of column col of s_nb.
-// vl_out (may be null): candidates within the list radius are appended to
-// the own particle's candidate list, vl_cnt counting them past kVlMax too.
 template <bool kBrute, bool kKnn, bool kF32, int kB, typename Src, typename Entry>
 __device__ __forceinline__ void list_batch(const DevParams &P, const Src &src, int (&b)[kB], int self, int oa,
                                            double xa, double ya, const F32Test &ft, Entry *s_nb, int col, int &cnt,
-                                           unsigned &my_pairs, int &my_nb, double &bx, double &by, double cd, int cj,
-                                           unsigned short *vl_out, int &vl_cnt)
+                                           unsigned &my_pairs, int &my_nb, double &bx, double &by, double cd, int cj)
 {
   constexpr Entry kRole = sizeof(Entry) == 2 ? (Entry)kRoleI16 : (Entry)kRoleI;
   bool sure[kB];  // FP32 says: surely inside and not coincident
@@ -280,10 +357,6 @@ __device__ __forceinline__ void list_batch(const DevParams &P, const Src &src, i
     for (int u = 0; u < kB; u++) {
       const float dxf = ft.xa - f[u].x, dyf = ft.ya - f[u].y;
       const float r2f = fmaf(dxf, dxf, dyf * dyf);
-      if (vl_out && b[u] != self && r2f < ft.vl) {
-        if (vl_cnt < kVlMax) vl_out[vl_cnt] = (unsigned short)b[u];
-        vl_cnt++;
-      }
       if (r2f > ft.hi) b[u] = self;  // surely outside: drop
       sure[u] = r2f < ft.lo && r2f > ft.tiny;
     }
@@ -333,12 +406,10 @@ __device__ __forceinline__ void list_batch(const DevParams &P, const Src &src, i
 // kKnn: the reference's k-nearest cap (DevParams::knn): a pair is kept iff
 // the partner is among query i's kept points -- the own particle's cut
 // (cd, cj) when it is i, the partner's (src.cut(b)) when the partner is i.
-// vl_out, vl_cnt: the candidate list written meanwhile (list_batch).
 template <bool kBrute, int kChunk, bool kKnn, bool kF32, typename Src, typename Cursor, typename Entry>
 __device__ __forceinline__ int tile_list(const DevParams &P, const Src &src, Cursor &cur, bool &more, int self,
                                         int oa, double xa, double ya, const F32Test &ft, Entry *s_nb, int col,
-                                        unsigned &my_pairs, int &my_nb, double &bx, double &by, double cd, int cj,
-                                        unsigned short *vl_out, int &vl_cnt)
+                                        unsigned &my_pairs, int &my_nb, double &bx, double &by, double cd, int cj)
 {
   constexpr int kB = 4;
   int cnt = 0;
@@ -353,36 +424,13 @@ __device__ __forceinline__ int tile_list(const DevParams &P, const Src &src, Cur
 #pragma unroll
     for (int u = 0; u < kB; u++) b[u] = (u < n) ? cur.at(pos + u) : self;
     list_batch<kBrute, kKnn, kF32, kB>(P, src, b, self, oa, xa, ya, ft, s_nb, col, cnt, my_pairs, my_nb, bx, by, cd,
-                                       cj, vl_out, vl_cnt);
-  }
-  return cnt;
-}
-
-// The listing from the own particle's candidate list, which the caller has
-// copied into rows 0 .. nshort - 1 of column col of s_nb: filtered in place
-// (a listed partner is written at a row not above the one it was read
-// from), in the list's order, which is the stencil walk's.  nshort <=
-// kVlMax <= the rows of s_nb.
-template <bool kBrute, bool kKnn, typename Src, typename Entry>
-__device__ __forceinline__ int tile_list_short(const DevParams &P, const Src &src, int nshort, int self, int oa,
-                                              double xa, double ya, const F32Test &ft, Entry *s_nb, int col,
-                                              unsigned &my_pairs, int &my_nb, double &bx, double &by, double cd,
-                                              int cj)
-{
-  constexpr int kB = 4;
-  int cnt = 0, none = 0;
-  for (int j = 0; j < nshort; j += kB) {
-    int b[kB];
-#pragma unroll
-    for (int u = 0; u < kB; u++) b[u] = (j + u < nshort) ? (int)s_nb[(j + u) * kTileThreads + col] : self;
-    list_batch<kBrute, kKnn, true, kB>(P, src, b, self, oa, xa, ya, ft, s_nb, col, cnt, my_pairs, my_nb, bx, by, cd,
-                                       cj, nullptr, none);
+                                       cj);
   }
   return cnt;
 }
 
 // A pass CTA's statistics: warp reductions, then one atomic per warp into
-// the counters the cell-list launch zeroed.
+// the counters zeroed before the pass.
 __device__ __forceinline__ void pass_stats(const PassStats &st, unsigned my_pairs, int my_nb)
 {
   const unsigned wp = __reduce_add_sync(0xffffffffu, my_pairs);

@@ -91,6 +91,7 @@ struct DevParams {
   int gravity_flag;
   double mu0, kappa, eps;
   double two_mu0;  // 2 mu0
+  double gamma4;   // 4 gamma
   int stress_type;
   int boundary_force;
   double k_spring, c_damp, dx, dy;
@@ -107,6 +108,7 @@ struct DevParams {
   int ncx, ncy;  // cells per axis, multiples of `tile`
   int tile;      // storage-order tile edge in cells
   int ntx;       // tiles per row
+  int lanes;     // lanes per particle of a step's pass (tile_stream.cuh): 1, 2 or 4
   int reach;     // cells are >= radius / reach wide; partners lie within `reach` cells
   // k-nearest cap of the reference's search (derivatives.c:1085 passes 40):
   // 0 = every in-radius pair; else each fluid query s keeps its knn nearest
@@ -178,6 +180,24 @@ struct WallTable {
 
 constexpr int kGridWords = 2;
 
+// What the recording pass after a cell-list build leaves for the passes
+// that stream tiles (tile_stream.cuh): the recorded tiles 0 .. *nstream - 1
+// (at most cap of them), and the hard ones that do not fit a stream.
+// A stream buffer holds kStreamCap records: two buffers of 112-byte records
+// (109 KB) for each of two CTAs fill an SM's shared memory; a lattice tile of
+// 11 cells at h = 1.3 dx has 420 to 441.
+constexpr int kStreamCap = 488;
+struct StreamTiles {
+  int *nstream, *nhard;  // reset by every build that rebuilds the list
+  unsigned *recorded;    // the list generation the record below belongs to
+  int *slot;             // [cap][kStreamCap] slots of the block's records, -1 past its end
+  int2 *core;            // [cap][kTileThreads] (slot, record) of each core particle, slot -1 for none
+  int *tile;             // [cap] storage tile
+  int *hard;             // [number of tiles] storage tiles
+  int *nlive, *live;     // the tiles that hold a particle at the last build, [number of tiles]
+  int cap;
+};
+
 struct CellGrid {
   int ncell;
   int *count;    // [ncell]
@@ -193,19 +213,20 @@ struct CellGrid {
   int *rank;       // [n]
   int *totals;     // [kCellBuildMaxBlocks + 1]
   unsigned *bar;   // [kGridWords]
-  // The tiled passes' candidate lists (the simulation's main grid only; null
-  // on other grids).  gen counts the builds that rebuilt the list.  A tile
-  // whose tile_gen equals gen has, for each of its fluid particles (by
-  // slot), vl_n candidates in vl[slot * kVlMax ...]: the records of its
-  // block within the list radius (the search radius plus twice the largest
-  // displacement a rebuild allows), in the stencil walk's order, or vl_n ==
-  // kVlOverflow when there were more than kVlMax.
+  // The tiled passes' candidate lists and recorded tiles (the simulation's
+  // main grid only; null on other grids).  gen counts the builds that rebuilt
+  // the list; the recording pass after a build writes, for each fluid
+  // particle (by slot), vl_n candidates in vl (the layout of CandWriter): the
+  // records of its tile's block within the list radius (the search radius
+  // plus twice the largest displacement a rebuild allows), in the stencil
+  // walk's order, or vl_n == kVlOverflow when there were more than vl_cap.
   unsigned *gen;           // [1]
-  unsigned *tile_gen;      // [number of tiles]
-  unsigned short *vl;      // [nf * kVlMax]
+  unsigned short *vl;      // [vl_cap * nf], vl_cap a multiple of 8
   unsigned char *vl_n;     // [nf]
+  int vl_cap;
+  StreamTiles st;
 };
-constexpr int kVlMax = 24;
+constexpr int kVlCapMax = 240;  // vl_n is a byte
 constexpr unsigned char kVlOverflow = 255;
 
 // Statistics of a rate pass, zeroed by the cell-list launch before it: pairs
@@ -277,6 +298,13 @@ struct StepOut {
 // (tile_pass.cuh); the cell list must be current.
 uph_status launch_ref_pass(const DevParams &P, const SlotArrays &S, const CellGrid &G, PassStats st,
                            const StepOut &F, cudaStream_t s);
+// The same for a step of uph_sim_step, the cell list included, in one launch
+// (tile_stream.cuh).
+struct StepArgs;
+uph_status launch_ref_step(const DevParams &P, const SlotArrays &S, const CellGrid &G, const StepOut &F,
+                           const StepArgs &A, unsigned *err, cudaStream_t s);
+uph_status launch_wcsph_step(const DevParams &P, const SlotArrays &S, const CellGrid &G, const StepOut &F,
+                             const StepArgs &A, unsigned *err, cudaStream_t s);
 // the REF profile's particle-packing pass (flag_init_simul == 0) in its place
 uph_status launch_packing_pass(const DevParams &P, const SlotArrays &S, const CellGrid &G, PassStats st,
                                cudaStream_t s);

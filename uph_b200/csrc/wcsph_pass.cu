@@ -19,8 +19,7 @@
 //
 // Execution as in the REF pass: a cheap listing phase (distance test only)
 // per thread into shared memory, then the pair arithmetic over the lists.
-#include "leapfrog.cuh"
-#include "tile_pass.cuh"
+#include "tile_stream.cuh"
 
 namespace uph {
 
@@ -32,11 +31,11 @@ __device__ __forceinline__ void wcsph_wall_pair(const DevParams &P, int itb, dou
   if (P.boundary_force == 3 && (itb == 2 || itb == 3 || itb == 5)) {
     const double r0 = 3.0 * P.dx;
     if (rr < r0) {
-      const double rv = dxd * dud + dyd * dvd;
+      const double rv = fma(dxd, dud, dyd * dvd);
       const double c1 = P.k_spring * (r0 - rr) / (rr * ma);
       const double c2 = P.c_damp * rv / (rr * rr * ma);
-      wx -= c1 * dxd + c2 * dxd;
-      wy -= c1 * dyd + c2 * dyd;
+      wx -= fma(c1, dxd, c2 * dxd);
+      wy -= fma(c1, dyd, c2 * dyd);
     }
   } else if (P.boundary_force == 4 && (itb == 2 || itb == 3) && rr < P.dx) {
     const double norm = 7.0 / (64.0 * 3.142 * P.h * P.h);
@@ -126,9 +125,11 @@ struct WcAcc {
 };
 
 // the sums of one pair (a, b), a = the own particle
-template <typename Real>
-__device__ __forceinline__ void wc_pair(const DevParams &P, const WcRec<Real> &a, const WcRec<Real> &b, bool isI,
-                                        Real &drho, Real &ax, Real &ay, WcAcc &W)
+// (the wall forces apart).  kMasked: a pair that is not `on` contributes
+// zeros (its kernel gradient is zero) instead of being branched around.
+template <bool kMasked, typename Real, typename Rec>
+__device__ __forceinline__ void wc_pair(const DevParams &P, const Rec &a, const Rec &b, bool on, Real &drho, Real &ax,
+                                        Real &ay)
 {
   const Real h = (Real)P.h, inv_h = (Real)P.inv_h, inv_h2 = (Real)P.inv_h2;
   const Real sigma = (Real)P.cs_alpha;
@@ -149,7 +150,7 @@ __device__ __forceinline__ void wc_pair(const DevParams &P, const WcRec<Real> &a
     dv = a.v - b.v;
     mb = b.m;
   }
-  const Real r2 = dx * dx + dy * dy;
+  const Real r2 = fma(dx, dx, dy * dy);
   if constexpr (sizeof(Real) == sizeof(float)) {
     inv_r = r2 > 0.0f ? rsqrtf(r2) : 0.0f;
     r = r2 * inv_r;
@@ -159,7 +160,7 @@ __device__ __forceinline__ void wc_pair(const DevParams &P, const WcRec<Real> &a
   const Real q = r * inv_h;
   Real F;
   if (q < (Real)1) {
-    F = sigma * ((Real)-3 + (Real)2.25 * q) * inv_h2;
+    F = sigma * fma((Real)2.25, q, (Real)-3) * inv_h2;
   } else {
     const Real t = (Real)2 - q;
     if constexpr (sizeof(Real) == sizeof(float))
@@ -167,9 +168,10 @@ __device__ __forceinline__ void wc_pair(const DevParams &P, const WcRec<Real> &a
     else
       F = -sigma * 0.75 * t * t * inv_h * rcp_nr(r);
   }
+  if (kMasked && !on) F = (Real)0;
   const Real gx = F * dx, gy = F * dy;
-  drho += mb * (du * gx + dv * gy);
-  const Real vr = du * dx + dv * dy;
+  drho = fma(mb, fma(du, gx, dv * gy), drho);
+  const Real vr = fma(du, dx, dv * dy);
   Real pi_ab = 0;
   if (vr < (Real)0) {
     if constexpr (sizeof(Real) == sizeof(float)) {
@@ -180,62 +182,55 @@ __device__ __forceinline__ void wc_pair(const DevParams &P, const WcRec<Real> &a
       pi_ab = -ac * mu * rcp_nr(0.5 * (a.rho + b.rho));
     }
   }
-  const Real pij = a.A1 + b.A1 + pi_ab;
-  ax -= mb * pij * gx;
-  ay -= mb * pij * gy;
-  if (isI && a.itype == 1 && b.itype >= 2) {
-    const double dxd = a.x - b.x, dyd = a.y - b.y;
-    wcsph_wall_pair(P, b.itype, exact_r2(dxd, dyd), dxd, dyd, a.u - b.u, a.v - b.v, a.m, W.wx, W.wy);
-  }
+  const Real mp = mb * (a.A1 + b.A1 + pi_ab);
+  ax = fma(-mp, gx, ax);
+  ay = fma(-mp, gy, ay);
 }
 
-// nshort, vl_out, vl_cnt: the candidate lists, as in the REF pass's
-// ref_particle
+// a listed pair's wall force: its i side is this fluid particle, its j side a wall
+template <typename Rec>
+__device__ __forceinline__ void wc_wall(const DevParams &P, const Rec &a, const Rec &b, WcAcc &W)
+{
+  const double dxd = a.x - b.x, dyd = a.y - b.y;
+  wcsph_wall_pair(P, b.itype, exact_r2(dxd, dyd), dxd, dyd, a.u - b.u, a.v - b.v, a.m, W.wx, W.wy);
+}
+
+// The stencil walk of one own particle, as in the REF pass's ref_particle.
 template <bool kBrute, bool kF32, typename Real, typename Src, typename Cursor, typename Entry>
 __device__ __forceinline__ void wc_particle(const DevParams &P, const Src &src, Cursor &cur, bool active, int self,
                                             const WcRec<Real> &o, const F32Test &ft, Entry *s_nb, Real &drho,
-                                            Real &ax, Real &ay, WcAcc &W, unsigned &my_pairs, int &my_nb, int nshort,
-                                            unsigned short *vl_out, int &vl_cnt)
+                                            Real &ax, Real &ay, WcAcc &W, unsigned &my_pairs, int &my_nb)
 {
   constexpr Entry kRole = sizeof(Entry) == 2 ? (Entry)kRoleI16 : (Entry)kRoleI;
   const int col = threadIdx.x;
   bool more = active;
   while (__any_sync(0xffffffffu, more)) {
-    int cnt = 0;
-    if (kF32 && nshort >= 0) {
-      if constexpr (kF32) {
-        if (more)
-          cnt = tile_list_short<kBrute, false>(P, src, nshort, self, o.orig, o.x, o.y, ft, s_nb, col, my_pairs, my_nb,
-                                               W.wx, W.wy, 0.0, 0);
-      }
-      more = false;
-    } else {
-      cnt = tile_list<kBrute, kTileChunk, false, kF32>(P, src, cur, more, self, o.orig, o.x, o.y, ft, s_nb, col,
-                                                       my_pairs, my_nb, W.wx, W.wy, 0.0, 0, vl_out, vl_cnt);
-    }
+    const int cnt = tile_list<kBrute, kTileChunk, false, kF32>(P, src, cur, more, self, o.orig, o.x, o.y, ft, s_nb, col,
+                                                               my_pairs, my_nb, W.wx, W.wy, 0.0, 0);
     __syncwarp();
     for (int e = 0; e < cnt; e++) {
       const Entry ent = s_nb[e * kTileThreads + col];
       const WcRec<Real> b = src.get((int)(ent & (Entry)~kRole));
-      wc_pair<Real>(P, o, b, (ent & kRole) != 0, drho, ax, ay, W);
+      wc_pair<false, Real>(P, o, b, true, drho, ax, ay);
+      if ((ent & kRole) != 0 && o.itype == 1 && b.itype >= 2) wc_wall(P, o, b, W);
     }
     __syncwarp();
   }
 }
 
 // dv/dt with the wall forces, gravity and the sponge layer
-template <typename Real>
-__device__ __forceinline__ void wc_accel(const DevParams &P, const SlotArrays &S, int a, const WcRec<Real> &o, Real ax,
+template <typename Real, typename Rec>
+__device__ __forceinline__ void wc_accel(const DevParams &P, const SlotArrays &S, int a, const Rec &o, Real ax,
                                          Real ay, const WcAcc &W, double &axd, double &ayd)
 {
   axd = (double)ax + W.wx;
   ayd = (double)ay + W.wy;
   if (P.gravity_flag == 1) ayd -= P.g;
-  if (P.moving_boundary == 1 && P.wave_absorption == 1) axd -= S.sponge[a] * o.u;
+  if (P.moving_boundary == 1 && P.wave_absorption == 1) axd = fma(-S.sponge[a], o.u, axd);
 }
 
-template <typename Real>
-__device__ __forceinline__ void wc_epilogue(const DevParams &P, const SlotArrays &S, int a, const WcRec<Real> &o,
+template <typename Real, typename Rec>
+__device__ __forceinline__ void wc_epilogue(const DevParams &P, const SlotArrays &S, int a, const Rec &o,
                                             Real drho, Real ax, Real ay, const WcAcc &W)
 {
   double axd, ayd;
@@ -262,9 +257,9 @@ __device__ __forceinline__ void wc_epilogue(const DevParams &P, const SlotArrays
 // other buffer.  Rates and the algebraic pressure are stored only by the
 // last step of a call, and the particle's constants not at all (see the REF
 // pass's ref_step_epilogue).
-template <typename Real>
+template <typename Real, typename Rec>
 __device__ __forceinline__ void wc_step_epilogue(const DevParams &P, const SlotArrays &S, const StepOut &F, int a,
-                                                 const WcRec<Real> &o, Real drho, Real ax, Real ay, const WcAcc &W)
+                                                 const Rec &o, Real drho, Real ax, Real ay, const WcAcc &W)
 {
   const SlotArrays &D = F.D;
   double axd, ayd;
@@ -360,12 +355,8 @@ __device__ __forceinline__ void wc_tile(const DevParams &P, const SlotArrays &S,
   if (ncore == 0) return;
   const bool staged = B.nrec <= kWcRecCap;
   // the origin of the block: FP32 positions are taken relative to it
-  const double ox = P.lo_x + B.bx0 * P.cell, oy = P.lo_y + B.by0 * P.cell;
+  const double ox = fma((double)B.bx0, P.cell, P.lo_x), oy = fma((double)B.by0, P.cell, P.lo_y);
   if (staged) {
-    // this tile's candidate lists are current if written since the last
-    // build (G.vl null: the lists are off, every particle walks the stencil)
-    const unsigned gen = G.vl ? *G.gen : 0u;
-    const bool vl_use = G.vl && G.tile_gen[tile] == gen;
     // two records per thread at a time, every load issued before the first
     // store (two rounds of loads: the slots, then their fields)
     for (int k0 = threadIdx.x; k0 < B.nrec; k0 += 2 * kTileThreads) {
@@ -373,18 +364,6 @@ __device__ __forceinline__ void wc_tile(const DevParams &P, const SlotArrays &S,
       const bool two = k1 < B.nrec;
       const int s0 = G.list[tile_record_pos(B, k0)];
       const int s1 = two ? G.list[tile_record_pos(B, k1)] : s0;
-      // the candidate lists the core's fluid particles will read after the
-      // staging: fetched into L2 meanwhile (the halo's too, for their tiles)
-      if (vl_use) {
-        if (s0 < P.nf) {
-          prefetch_l2(G.vl + (size_t)s0 * kVlMax);
-          prefetch_l2(G.vl_n + s0);
-        }
-        if (two && s1 < P.nf) {
-          prefetch_l2(G.vl + (size_t)s1 * kVlMax);
-          prefetch_l2(G.vl_n + s1);
-        }
-      }
       const WcRec<Real> r0 = load_wc_rec<Real>(S, s0, ox, oy);
       const WcRec<Real> r1 = load_wc_rec<Real>(S, s1, ox, oy);
       rec[k0] = r0;
@@ -416,16 +395,11 @@ __device__ __forceinline__ void wc_tile(const DevParams &P, const SlotArrays &S,
       StagedCursor cur;
       cur.c.init(B, P.reach, active ? cx : B.bx0, active ? cy : B.by0);
       const float2 of = s_posf[active ? kr : 0];
-      const F32Test ft = make_f32_test(P, B, of.x, of.y);
+      const F32Test ft = make_f32_test(P, max(B.W, B.H), of.x, of.y);
       Real drho = 0, ax = 0, ay = 0;
       WcAcc W = {0.0, 0.0};
       int nb = 0;
-      int nshort = -1, vl_cnt = 0;
-      unsigned short *vl_out = nullptr;
-      if (active && G.vl) nshort = load_candidates(G, a, vl_use, s_nb16, threadIdx.x, vl_out);
-      wc_particle<kBrute, true, Real>(P, src, cur, active, kr, o, ft, s_nb16, drho, ax, ay, W, my_pairs, nb, nshort,
-                                      vl_out, vl_cnt);
-      if (vl_out) G.vl_n[a] = vl_cnt <= kVlMax ? (unsigned char)vl_cnt : kVlOverflow;
+      wc_particle<kBrute, true, Real>(P, src, cur, active, kr, o, ft, s_nb16, drho, ax, ay, W, my_pairs, nb);
       my_nb = max(my_nb, nb);
       if (active) {
         if (F.enabled)
@@ -434,7 +408,6 @@ __device__ __forceinline__ void wc_tile(const DevParams &P, const SlotArrays &S,
           wc_epilogue<Real>(P, S, a, o, drho, ax, ay, W);
       }
     }
-    if (G.vl && !vl_use && threadIdx.x == 0) G.tile_gen[tile] = gen;
   } else {
     unsigned *s_nb32 = reinterpret_cast<unsigned *>(rec);
     const WcGlobalSrc<Real> src{S, ox, oy};
@@ -455,9 +428,7 @@ __device__ __forceinline__ void wc_tile(const DevParams &P, const SlotArrays &S,
       Real drho = 0, ax = 0, ay = 0;
       WcAcc W = {0.0, 0.0};
       int nb = 0;
-      int vl_none = 0;
-      wc_particle<kBrute, false, Real>(P, src, cur, active, as, o, ft, s_nb32, drho, ax, ay, W, my_pairs, nb, -1,
-                                       nullptr, vl_none);
+      wc_particle<kBrute, false, Real>(P, src, cur, active, as, o, ft, s_nb32, drho, ax, ay, W, my_pairs, nb);
       my_nb = max(my_nb, nb);
       if (active) {
         if (F.enabled)
@@ -513,6 +484,180 @@ uph_status launch_wcsph_pass(const DevParams &P, const SlotArrays &S, const Cell
   if (P.precision == UPH_PREC_FP32_PAIR)
     return brute ? launch_wc<true, float>(P, S, G, st, F, s) : launch_wc<false, float>(P, S, G, st, F, s);
   return brute ? launch_wc<true, double>(P, S, G, st, F, s) : launch_wc<false, double>(P, S, G, st, F, s);
+}
+
+// ---- a step in one launch (tile_stream.cuh) -------------------------------------------
+// One particle as the stream holds it: the state arrays' fields, p replaced
+// by p / rho^2 when its owner converts it.
+struct __align__(16) WcRaw {
+  double x, y, u, v, m, A1, rho, ir;
+  int itype, pad[3];
+};
+// FP32: the pair loop's operands beside it, as WcRec<float> holds them.
+struct __align__(16) WcRaw32 {
+  WcRaw d;
+  float xr, yr, ur, vr, mr, A1, rho, pad;
+};
+static_assert(sizeof(WcRaw) == 80 && sizeof(WcRaw32) == 112, "record strides of the stream");
+struct __align__(16) WcPair32 {  // the FP32 half
+  float xr, yr, ur, vr, mr, A1, rho, pad;
+};
+
+template <bool kBrute, typename Real>
+struct WcStream {
+  static constexpr bool kF32 = sizeof(Real) == sizeof(float);
+  static constexpr int kStride = kF32 ? sizeof(WcRaw32) : sizeof(WcRaw);
+  const DevParams &P;
+  const SlotArrays &S;
+  const StepOut &F;
+  unsigned my_pairs;
+  int my_nb;
+  float lo, hi, tiny;  // the FP32 pair test's thresholds (F32Test) for the widest block
+
+  __device__ __forceinline__ void stage(int s, uint32_t dst) const
+  {
+    const double *f[8] = {S.x, S.y, S.u, S.v, S.m, S.p, S.rho, S.inv_rho};
+#pragma unroll
+    for (int k = 0; k < 8; k++) cp_async8(dst + 8 * k, f[k] + s);
+    cp_async4(dst + 64, S.itype + s);
+  }
+  __device__ __forceinline__ void convert_one(unsigned char *p, double ox, double oy) const
+  {
+    WcRaw &r = *reinterpret_cast<WcRaw *>(p);
+    const double ir = r.ir;
+    if constexpr (kF32) {
+      WcRaw32 &q = *reinterpret_cast<WcRaw32 *>(p);
+      q.xr = (float)(r.x - ox);
+      q.yr = (float)(r.y - oy);
+      q.ur = (float)r.u;
+      q.vr = (float)r.v;
+      q.mr = (float)r.m;
+      q.A1 = (float)(r.A1 * ir * ir);
+      q.rho = (float)r.rho;
+    } else {
+      r.A1 = r.A1 * ir * ir;
+    }
+  }
+  // the records this thread copied (null: none); FP32: positions relative
+  // to the tile's block, as tile_setup places it
+  __device__ __forceinline__ void convert(int tile, unsigned char *p0, unsigned char *p1) const
+  {
+    double ox = 0.0, oy = 0.0;
+    if constexpr (kF32) {
+      const int bx0 = max((tile % P.ntx) * P.tile - P.reach, 0), by0 = max((tile / P.ntx) * P.tile - P.reach, 0);
+      ox = fma((double)bx0, P.cell, P.lo_x);
+      oy = fma((double)by0, P.cell, P.lo_y);
+    }
+    if (p0) convert_one(p0, ox, oy);
+    if (p1) convert_one(p1, ox, oy);
+  }
+  __device__ __forceinline__ void begin(int a) const
+  {
+    if (!F.enabled || a < 0 || (F.first_step && F.predict_next)) return;
+    prefetch_l2(S.rho_min + a);
+    prefetch_l2(S.p_min + a);
+    prefetch_l2(S.u_min + a);
+    prefetch_l2(S.v_min + a);
+  }
+  template <int kLanes, typename Stream>
+  __device__ __forceinline__ void particle(const unsigned char *buf, int rec, int a, int n, CandReader<kLanes> &rd,
+                                           Stream &stream)
+  {
+    const WcRaw own = *reinterpret_cast<const WcRaw *>(buf + (size_t)rec * kStride);
+    Real drho = 0, ax = 0, ay = 0;
+    WcAcc W = {0.0, 0.0};
+    int nb = 0;
+    const int most = max(__reduce_max_sync(0xffffffffu, n), Stream::kReadyAt + 1);
+    WcPair32 of = {};
+    if constexpr (kF32) of = *reinterpret_cast<const WcPair32 *>(buf + (size_t)rec * kStride + sizeof(WcRaw));
+    for (int e = 0; e < most; e++) {
+      stream.refill(e);
+      const unsigned c = rd.next(e);
+      const unsigned char *p = buf + (size_t)(e < n ? (int)(c & kCandRec) : rec) * kStride;
+      const WcRaw &d = *reinterpret_cast<const WcRaw *>(p);
+      bool in, near;
+      auto exact = [&]() {
+        const double r2 = exact_r2(own.x - d.x, own.y - d.y);
+        in = e < n && r2 < P.r2cut;
+        near = in && r2 > DBL_EPSILON;
+      };
+      WcPair32 bf = {};
+      if constexpr (kF32) {
+        bf = *reinterpret_cast<const WcPair32 *>(p + sizeof(WcRaw));
+        const float dxf = of.xr - bf.xr, dyf = of.yr - bf.yr;
+        const float r2f = fmaf(dxf, dxf, dyf * dyf);
+        // surely in or out by the FP32 distance; near the cut-off (or at a
+        // possible coincidence) by the exact FP64 one
+        in = e < n && r2f < lo;
+        near = in && r2f > tiny;
+        if (e < n && !near && !(r2f > hi)) exact();
+      } else {
+        exact();
+      }
+      if (kBrute && in && (c & kCandBoundary)) {
+        const double dx = own.x - d.x, dy = own.y - d.y;
+        brute_wall_force(P, exact_r2(dx, dy), dx, dy, d.m, W.wx, W.wy);
+      }
+      nb += near;
+      const bool on = near && !(c & kCandNoPair);
+      my_pairs += on && (c & kCandI);
+      if constexpr (kF32)
+        wc_pair<true, Real>(P, of, bf, on, drho, ax, ay);
+      else
+        wc_pair<true, Real>(P, own, d, on, drho, ax, ay);
+      if (on && (c & kCandWall)) wc_wall(P, own, d, W);
+    }
+    stream.done_reading();
+    if constexpr (kLanes > 1) {
+      drho = lanes_sum<kLanes>(drho);
+      ax = lanes_sum<kLanes>(ax);
+      ay = lanes_sum<kLanes>(ay);
+      W.wx = lanes_sum<kLanes>(W.wx);
+      W.wy = lanes_sum<kLanes>(W.wy);
+      nb = lanes_sum<kLanes>(nb);
+    }
+    my_nb = max(my_nb, nb);
+    if (a < 0 || (threadIdx.x & (kLanes - 1)) != 0) return;
+    if (F.enabled)
+      wc_step_epilogue<Real>(P, S, F, a, own, drho, ax, ay, W);
+    else
+      wc_epilogue<Real>(P, S, a, own, drho, ax, ay, W);
+  }
+};
+
+template <bool kBrute, int kLanes, typename Real>
+__global__ void __launch_bounds__(kTileThreads, 2) k_wcsph_step(const CellBuildArgs C, const SlotArrays S,
+                                                             const StepOut F, const StepArgs A)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const F32Test ft = make_f32_test(C.P, C.P.tile + 2 * C.P.reach, 0.f, 0.f);
+  WcStream<kBrute, Real> ps{C.P, S, F, 0u, 0, ft.lo, ft.hi, ft.tiny};
+  step_run<kBrute, kLanes>(C, S, F, A, ps, smem, [&](int tile) {
+    wc_tile<kBrute, Real>(C.P, S, C.G, F, tile, smem, ps.my_pairs, ps.my_nb);
+  });
+}
+
+template <bool kBrute, typename Real>
+uph_status launch_wc_step(const DevParams &P, const SlotArrays &S, const CellGrid &G, const StepOut &F,
+                          const StepArgs &A, unsigned *err, cudaStream_t s)
+{
+  constexpr size_t sm =
+      std::max({wc_smem<Real>(), stream_smem_bytes<WcStream<kBrute, Real>::kStride>(), kRecordSmemBytes});
+  if constexpr (sizeof(Real) == sizeof(double)) {
+    if (P.lanes == 4) return launch_step<k_wcsph_step<kBrute, 4, Real>>(sm, P, S, G, F, A, err, s);
+    if (P.lanes == 2) return launch_step<k_wcsph_step<kBrute, 2, Real>>(sm, P, S, G, F, A, err, s);
+  }
+  return launch_step<k_wcsph_step<kBrute, 1, Real>>(sm, P, S, G, F, A, err, s);
+}
+
+uph_status launch_wcsph_step(const DevParams &P, const SlotArrays &S, const CellGrid &G, const StepOut &F,
+                             const StepArgs &A, unsigned *err, cudaStream_t s)
+{
+  const bool brute = P.boundary_force != 3 && P.boundary_force != 4 && P.boundary_force != 5;
+  if (P.precision == UPH_PREC_FP32_PAIR)
+    return brute ? launch_wc_step<true, float>(P, S, G, F, A, err, s) : launch_wc_step<false, float>(P, S, G, F, A, err, s);
+  return brute ? launch_wc_step<true, double>(P, S, G, F, A, err, s)
+               : launch_wc_step<false, double>(P, S, G, F, A, err, s);
 }
 
 }  // namespace uph
