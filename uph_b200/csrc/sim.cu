@@ -81,7 +81,7 @@ struct uph_sim {
   // published by the step's launch, and that launch's running sums
   unsigned long long *d_niac = nullptr;
   int *d_max_nb = nullptr;
-  unsigned *d_step_done = nullptr, *d_moved = nullptr, *d_phases = nullptr;
+  unsigned *d_step_done = nullptr, *d_moved = nullptr, *d_ticket = nullptr, *d_phases = nullptr;
   int *d_perm = nullptr;  // scratch for uploads
   int itime = 0;
   int steps_since_reorder = 0;
@@ -97,6 +97,8 @@ struct uph_sim {
   double fam_ms[KF_COUNT] = {0};
   int64_t fam_launch[KF_COUNT] = {0};
   std::vector<void *> allocations;
+  void *grid_block = nullptr, *stream_block = nullptr;  // the per-cell arrays; the stream's per-tile arrays
+  bool search_only = false;
   double *d_partials = nullptr;
   int n_partials = 0;
   // device step counter (steps completed) and moving-wall table
@@ -141,36 +143,54 @@ struct uph_sim {
   int *pe_cnt = nullptr, *pe_off = nullptr, *pe_bsum = nullptr;
   int32_t *pe_ip = nullptr, *pe_jp = nullptr;
   double *pe_r2 = nullptr, *pe_w = nullptr, *pe_dw = nullptr;
-  int64_t pe_cap = 0;
+  int64_t pe_cap = 0, pe_kernel_cap = 0;
+  void *pe_index = nullptr, *pe_block = nullptr, *pe_kernel = nullptr;  // counts; i, j, rij2; w, dwcdx
   bool kcut_fresh = false;  // the knn cut matches the current positions and cell list
 };
 
 namespace {
 
-template <typename T>
-cudaError_t dalloc(uph_sim *s, T **p, size_t count)
-{
-  *p = nullptr;
-  if (count == 0) count = 1;
-  cudaError_t e = cudaMalloc((void **)p, sizeof(T) * count);
-  if (e == cudaSuccess) s->allocations.push_back((void *)*p);
-  return e;
-}
+// One device allocation for many arrays: `want` notes where an array's
+// address goes, `commit` allocates the block and fills the addresses in (256
+// bytes apart at least).  An allocation costs about 0.6 ms whatever its size,
+// and a simulation has over a hundred arrays (64 ms to create one with an
+// allocation each).
+struct Block {
+  std::vector<std::pair<void **, size_t>> wanted;
 
-cudaError_t alloc_slots(uph_sim *s, SlotArrays &A, int n, int nf)
+  template <typename T>
+  void want(T **p, size_t count)
+  {
+    *p = nullptr;
+    wanted.emplace_back(reinterpret_cast<void **>(p), sizeof(T) * std::max<size_t>(count, 1));
+  }
+  cudaError_t commit(void **base)
+  {
+    size_t bytes = 0;
+    for (auto &w : wanted) bytes += (w.second + 255) & ~size_t(255);
+    *base = nullptr;
+    const cudaError_t e = cudaMalloc(base, bytes);
+    if (e != cudaSuccess) return e;
+    char *at = static_cast<char *>(*base);
+    for (auto &w : wanted) {
+      *w.first = at;
+      at += (w.second + 255) & ~size_t(255);
+    }
+    wanted.clear();
+    return cudaSuccess;
+  }
+};
+
+void want_slots(Block &B, SlotArrays &A, int n, int nf)
 {
-  cudaError_t e = cudaSuccess;
   double **all[] = {&A.x, &A.y, &A.u, &A.v, &A.ut, &A.vt, &A.rho, &A.rhot, &A.p, &A.pt, &A.m, &A.inv_rho,
                     &A.inv_rhot, &A.pressure};
-  for (double **p : all)
-    if ((e = dalloc(s, p, (size_t)n)) != cudaSuccess) return e;
-  if ((e = dalloc(s, &A.itype, (size_t)n)) != cudaSuccess) return e;
-  if ((e = dalloc(s, &A.orig, (size_t)n)) != cudaSuccess) return e;
+  for (double **p : all) B.want(p, (size_t)n);
+  B.want(&A.itype, (size_t)n);
+  B.want(&A.orig, (size_t)n);
   double **fl[] = {&A.rho_min, &A.p_min, &A.u_min, &A.v_min, &A.sponge, &A.drho, &A.dp, &A.ax, &A.ay,
                    &A.drho_a, &A.dp_a, &A.ax_a, &A.ay_a, &A.frho, &A.fp, &A.fu, &A.fv};
-  for (double **p : fl)
-    if ((e = dalloc(s, p, (size_t)nf)) != cudaSuccess) return e;
-  return cudaSuccess;
+  for (double **p : fl) B.want(p, (size_t)nf);
 }
 
 // adds the recorded event pairs to the per-family totals; the caller has
@@ -474,7 +494,7 @@ uph_status rate_pass(uph_sim *s, bool refresh, bool step = false, const StepOut 
   if (step && s->P.knn == 0 && s->P.nf > 0 &&
       (s->P.profile != UPH_PROFILE_REF || s->P.flag_init_simul == 1)) {
     Timer t(s, KF_PASS);
-    const StepArgs A{PassStats{s->d_niac + 1, s->d_max_nb + 1}, st, s->d_step_done, s->d_moved, s->d_step_done + 4, s->d_phases,
+    const StepArgs A{PassStats{s->d_niac + 1, s->d_max_nb + 1}, st, s->d_step_done, s->d_moved, s->d_ticket, s->d_phases,
                      s->cand_lists ? 0 : 1, s->d_itime};
     const StepOut out = F ? *F : StepOut{};
     r = s->P.profile != UPH_PROFILE_REF ? launch_wcsph_step(s->P, s->S, s->G, out, A, s->d_err, s->stream)
@@ -566,20 +586,20 @@ cudaError_t alloc_grid(uph_sim *s)
   // about 225 of them; one beyond the capacity is handled as a hard tile
   const long long ntiles = (long long)s->P.ntx * (s->P.ncy / s->P.tile);
   const long long want = std::min(ntiles, (long long)s->P.nf / 64 + 1024);
-  if (ntiles > s->stream_tiles) {
+  if (!s->search_only && ntiles > s->stream_tiles) {
     StreamTiles &t = G.st;
-    for (void *p : {(void *)t.slot, (void *)t.core, (void *)t.tile, (void *)t.hard, (void *)t.live})
-      if (p) cudaFree(p);
-    t.slot = t.tile = t.hard = t.live = nullptr;
-    t.core = nullptr;
+    if (s->stream_block) cudaFree(s->stream_block);
+    s->stream_block = nullptr;
     t.cap = 0;
     s->stream_tiles = 0;
-    cudaError_t e;
-    if ((e = cudaMalloc((void **)&t.slot, sizeof(int) * want * kStreamCap)) != cudaSuccess) return e;
-    if ((e = cudaMalloc((void **)&t.core, sizeof(int2) * want * kTileThreads)) != cudaSuccess) return e;
-    if ((e = cudaMalloc((void **)&t.tile, sizeof(int) * want)) != cudaSuccess) return e;
-    if ((e = cudaMalloc((void **)&t.hard, sizeof(int) * ntiles)) != cudaSuccess) return e;
-    if ((e = cudaMalloc((void **)&t.live, sizeof(int) * ntiles)) != cudaSuccess) return e;
+    Block B;
+    B.want(&t.slot, (size_t)want * kStreamCap);
+    B.want(&t.core, (size_t)want * kTileThreads);
+    B.want(&t.tile, (size_t)want);
+    B.want(&t.hard, (size_t)ntiles);
+    B.want(&t.live, (size_t)ntiles);
+    const cudaError_t e = B.commit(&s->stream_block);
+    if (e != cudaSuccess) return e;
     t.cap = (int)want;
     s->stream_tiles = ntiles;
   }
@@ -588,24 +608,25 @@ cudaError_t alloc_grid(uph_sim *s)
   // completed before the caller's next launch (a list build that started on
   // stale counts would scatter out of range)
   if (ncell <= s->grid_capacity) return cudaDeviceSynchronize();
-  for (int **p : {&G.count, &G.start, &G.fill, &G.block_sums, &s->gv.count, &s->gv.start, &s->gv.fill}) {
-    if (*p) cudaFree(*p);
-    *p = nullptr;
+  if (s->grid_block) cudaFree(s->grid_block);
+  s->grid_block = nullptr;
+  s->grid_capacity = 0;
+  Block B;
+  B.want(&G.count, (size_t)ncell);
+  B.want(&G.start, (size_t)ncell + 1);
+  B.want(&G.fill, (size_t)ncell);
+  B.want(&G.block_sums, (size_t)G.nblock_sums + 1);
+  CellGrid &V = s->gv;
+  if (s->P.nvrules > 0) {
+    B.want(&V.count, (size_t)ncell);
+    B.want(&V.start, (size_t)ncell + 1);
+    B.want(&V.fill, (size_t)ncell);
   }
-  cudaError_t e;
-  if ((e = cudaMalloc((void **)&G.count, sizeof(int) * ncell)) != cudaSuccess) return e;
-  if ((e = cudaMalloc((void **)&G.start, sizeof(int) * (ncell + 1))) != cudaSuccess) return e;
-  if ((e = cudaMalloc((void **)&G.fill, sizeof(int) * ncell)) != cudaSuccess) return e;
-  if ((e = cudaMalloc((void **)&G.block_sums, sizeof(int) * (G.nblock_sums + 1))) != cudaSuccess) return e;
+  cudaError_t e = B.commit(&s->grid_block);
+  if (e != cudaSuccess) return e;
   // the one-launch build keeps count all zero between builds
   if ((e = cudaMemset(G.count, 0, sizeof(int) * ncell)) != cudaSuccess) return e;
-  if (s->P.nvrules > 0) {
-    CellGrid &V = s->gv;
-    if ((e = cudaMalloc((void **)&V.count, sizeof(int) * ncell)) != cudaSuccess) return e;
-    if ((e = cudaMalloc((void **)&V.start, sizeof(int) * (ncell + 1))) != cudaSuccess) return e;
-    if ((e = cudaMalloc((void **)&V.fill, sizeof(int) * ncell)) != cudaSuccess) return e;
-    if ((e = cudaMemset(V.count, 0, sizeof(int) * ncell)) != cudaSuccess) return e;
-  }
+  if (s->P.nvrules > 0 && (e = cudaMemset(V.count, 0, sizeof(int) * ncell)) != cudaSuccess) return e;
   s->grid_capacity = ncell;
   return cudaDeviceSynchronize();
 }
@@ -807,7 +828,10 @@ DevParams make_dev_params(const uph_params *p)
 
 // ---- C ABI ---------------------------------------------------------------------
 
-extern "C" uph_status uph_sim_create(const uph_params *p, uph_sim **out)
+namespace {
+// search_only: a simulation that only finds pairs (uph_search_neighbors), with
+// no state but positions
+uph_status create_sim(const uph_params *p, uph_sim **out, bool search_only)
 {
   if (!p || !out) return fail(UPH_BAD_ARG, "uph_sim_create: NULL argument");
   *out = nullptr;
@@ -833,111 +857,123 @@ extern "C" uph_status uph_sim_create(const uph_params *p, uph_sim **out)
       return cuda_fail(e_, #x);      \
     }                                \
   } while (0)
-  TRY(alloc_slots(s, s->S, n, nf));
-  TRY(alloc_slots(s, s->S2, n, nf));
+  s->search_only = search_only;
   CellGrid &G = s->G;
-  TRY(dalloc(s, &G.list, (size_t)n));
-  TRY(dalloc(s, &G.cell_of, (size_t)n));
+  Staging &T = s->T;
+  Block B;
+  B.want(&G.list, (size_t)n);
+  B.want(&G.cell_of, (size_t)n);
+  B.want(&G.rank, (size_t)n);
+  B.want(&G.totals, (size_t)kCellBuildMaxBlocks + 1);
+  B.want(&G.bar, kGridWords);
+  B.want(&G.gen, 1);
+  B.want(&s->P.xbin, (size_t)n);
+  B.want(&s->P.ybin, (size_t)n);
+  B.want(&s->P.rebuild, 1);
+  B.want(&T.pos, 2 * (size_t)n);
+  B.want(&s->d_err, 1);
   if (s->P.knn > 0) {
-    TRY(dalloc(s, &s->P.kcut_d2, (size_t)nf));
-    TRY(dalloc(s, &s->P.kcut_j, (size_t)nf));
+    B.want(&s->P.kcut_d2, (size_t)nf);
+    B.want(&s->P.kcut_j, (size_t)nf);
   }
-  if (s->P.stress_type == 2 && s->P.profile == UPH_PROFILE_REF) {
-    TRY(dalloc(s, &s->P.str_xx, (size_t)n));
-    TRY(dalloc(s, &s->P.str_xy, (size_t)n));
-    TRY(dalloc(s, &s->P.str_yy, (size_t)n));
-  }
-  {
-    double *m0 = nullptr;
-    TRY(dalloc(s, &m0, 1));
-    TRY(cudaMemset(m0, 0, sizeof(double)));
-    s->P.pack_mass0 = m0;
-  }
-  TRY(dalloc(s, &s->P.xbin, (size_t)n));
-  TRY(dalloc(s, &s->P.ybin, (size_t)n));
-  TRY(dalloc(s, &s->P.rebuild, 1));
-  TRY(cudaMemset(s->P.rebuild, 1, sizeof(unsigned)));
-  TRY(dalloc(s, &G.gen, 1));
-  TRY(cudaMemset(G.gen, 0, sizeof(unsigned)));
-  {
+  // nstream, nhard, recorded, nlive; the step's finished blocks, skin flag,
+  // tile ticket and build phases
+  int *words = nullptr;
+  constexpr int kWords = 8 + 2 * TicketPhases::kPhases;
+  B.want(&words, kWords);
+  double *mass0 = nullptr;
+  VirtualBuf &V = s->vb;
+  CellGrid &Gv = s->gv;
+  const size_t nm = p->n_moving > 0 ? p->n_moving : 1;
+  if (search_only) {
+    B.want(&s->S.x, (size_t)n);
+    B.want(&s->S.y, (size_t)n);
+    B.want(&s->S.orig, (size_t)n);
+  } else {
+    want_slots(B, s->S, n, nf);
+    want_slots(B, s->S2, n, nf);
+    if (s->P.stress_type == 2 && s->P.profile == UPH_PROFILE_REF) {
+      B.want(&s->P.str_xx, (size_t)n);
+      B.want(&s->P.str_xy, (size_t)n);
+      B.want(&s->P.str_yy, (size_t)n);
+    }
+    B.want(&mass0, 1);
     // room for 1.3 times the candidates of a lattice (pi (R_l / dx)^2, R_l
     // the list radius), so that moving water seldom overflows: 32 entries at
     // h = 1.3 dx
     const double Rl = sqrt(s->P.r2cut) + 2.0 * 1.4142135623730951 * s->P.skin;
     const double want = 1.3 * 3.14159 * (Rl / p->dx) * (Rl / p->dx);
     G.vl_cap = want >= kVlCapMax ? kVlCapMax : std::max(16, (int)ceil(want / 8.0) * 8);
-  }
-  TRY(dalloc(s, &G.vl, (size_t)nf * G.vl_cap));
-  {
-    int *w = nullptr;  // nstream, nhard, recorded, nlive; the step's finished blocks, skin flag, tile ticket and build phases
-    constexpr int kWords = 8 + 2 * TicketPhases::kPhases;
-    TRY(dalloc(s, &w, kWords));
-    TRY(cudaMemset(w, 0, kWords * sizeof(int)));
-    G.st.nstream = w;
-    G.st.nhard = w + 1;
-    G.st.recorded = reinterpret_cast<unsigned *>(w + 2);
-    s->d_step_done = reinterpret_cast<unsigned *>(w + 3);
-    s->d_moved = reinterpret_cast<unsigned *>(w + 4);
-    G.st.nlive = w + 5;
-    s->d_phases = reinterpret_cast<unsigned *>(w + 8);
-  }
-  TRY(dalloc(s, &G.vl_n, (size_t)nf));
-  TRY(dalloc(s, &G.rank, (size_t)n));
-  TRY(dalloc(s, &G.totals, (size_t)kCellBuildMaxBlocks + 1));
-  TRY(dalloc(s, &G.bar, kGridWords));
-  TRY(cudaMemset(G.bar, 0, kGridWords * sizeof(unsigned)));
-  if (s->P.nvrules > 0) {
-    VirtualBuf &V = s->vb;
-    V.cap = s->P.nvrules * nf;
-    TRY(dalloc(s, &V.flags, (size_t)V.cap));
-    TRY(dalloc(s, &V.offs, (size_t)V.cap));
-    TRY(dalloc(s, &V.block_sums, (size_t)scan_block_sums_needed(V.cap) + 1));
-    TRY(dalloc(s, &V.count, 1));
-    TRY(cudaMemset(V.count, 0, sizeof(int)));
-    TRY(dalloc(s, &V.x, (size_t)V.cap));
-    TRY(dalloc(s, &V.y, (size_t)V.cap));
-    TRY(dalloc(s, &V.src, (size_t)V.cap));
-    TRY(dalloc(s, &V.rule, (size_t)V.cap));
-    CellGrid &Gv = s->gv;
-    TRY(dalloc(s, &Gv.list, (size_t)V.cap));
-    TRY(dalloc(s, &Gv.cell_of, (size_t)V.cap));
-    TRY(dalloc(s, &Gv.rank, (size_t)V.cap));
-    TRY(dalloc(s, &Gv.totals, (size_t)kCellBuildMaxBlocks + 1));
-    TRY(dalloc(s, &Gv.bar, kGridWords));
-    TRY(cudaMemset(Gv.bar, 0, kGridWords * sizeof(unsigned)));
-  }
-  TRY(alloc_grid(s));
-  Staging &T = s->T;
-  double **tall[] = {&T.rho, &T.lrho, &T.p, &T.lp, &T.mass, &T.pressure, &T.tmp_x, &T.tmp_y};
-  for (double **q : tall) TRY(dalloc(s, q, (size_t)n));
-  double **tall2[] = {&T.pos, &T.vel, &T.lvel};
-  for (double **q : tall2) TRY(dalloc(s, q, 2 * (size_t)n));
-  TRY(dalloc(s, &T.itype, (size_t)n));
-  double **tfl[] = {&T.rhomin, &T.pmin, &T.sponge, &T.drho, &T.dp, &T.drho_a, &T.dp_a, &T.frho, &T.fp};
-  for (double **q : tfl) TRY(dalloc(s, q, (size_t)nf));
-  double **tfl2[] = {&T.vmin, &T.acc, &T.acc_a, &T.fvel};
-  for (double **q : tfl2) TRY(dalloc(s, q, 2 * (size_t)nf));
-  TRY(dalloc(s, &s->d_err, 1));
-  TRY(dalloc(s, &s->d_niac, 2));  // the last pass's; a step's running sums
-  TRY(dalloc(s, &s->d_max_nb, 2));
-  TRY(cudaMemset(s->d_niac, 0, 2 * sizeof(unsigned long long)));
-  TRY(cudaMemset(s->d_max_nb, 0, 2 * sizeof(int)));
-  TRY(dalloc(s, &s->d_perm, (size_t)n));
-  TRY(dalloc(s, &s->d_itime, 1));
-  TRY(dalloc(s, &s->d_wall_tab, 4 * (size_t)(p->n_moving > 0 ? p->n_moving : 1)));
-  s->W.base = s->d_wall_tab + 3 * (size_t)(p->n_moving > 0 ? p->n_moving : 1);
-  s->n_partials = 1024;
-  TRY(dalloc(s, &s->d_partials, (size_t)s->n_partials * 4));
-  {
+    B.want(&G.vl, (size_t)nf * G.vl_cap);
+    B.want(&G.vl_n, (size_t)nf);
+    if (s->P.nvrules > 0) {
+      V.cap = s->P.nvrules * nf;
+      B.want(&V.flags, (size_t)V.cap);
+      B.want(&V.offs, (size_t)V.cap);
+      B.want(&V.block_sums, (size_t)scan_block_sums_needed(V.cap) + 1);
+      B.want(&V.count, 1);
+      B.want(&V.x, (size_t)V.cap);
+      B.want(&V.y, (size_t)V.cap);
+      B.want(&V.src, (size_t)V.cap);
+      B.want(&V.rule, (size_t)V.cap);
+      B.want(&Gv.list, (size_t)V.cap);
+      B.want(&Gv.cell_of, (size_t)V.cap);
+      B.want(&Gv.rank, (size_t)V.cap);
+      B.want(&Gv.totals, (size_t)kCellBuildMaxBlocks + 1);
+      B.want(&Gv.bar, kGridWords);
+    }
+    double **tall[] = {&T.rho, &T.lrho, &T.p, &T.lp, &T.mass, &T.pressure, &T.tmp_x, &T.tmp_y};
+    for (double **q : tall) B.want(q, (size_t)n);
+    B.want(&T.vel, 2 * (size_t)n);
+    B.want(&T.lvel, 2 * (size_t)n);
+    B.want(&T.itype, (size_t)n);
+    double **tfl[] = {&T.rhomin, &T.pmin, &T.sponge, &T.drho, &T.dp, &T.drho_a, &T.dp_a, &T.frho, &T.fp};
+    for (double **q : tfl) B.want(q, (size_t)nf);
+    double **tfl2[] = {&T.vmin, &T.acc, &T.acc_a, &T.fvel};
+    for (double **q : tfl2) B.want(q, 2 * (size_t)nf);
+    B.want(&s->d_perm, (size_t)n);
+    B.want(&s->d_wall_tab, 4 * nm);
+    s->n_partials = 1024;
+    B.want(&s->d_partials, (size_t)s->n_partials * 4);
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int want = (p->n_fluid + 255) / 256;
-    s->diag_blocks = want < 2 * sms ? (want > 0 ? want : 1) : 2 * sms;
+    const int want_blocks = (p->n_fluid + 255) / 256;
+    s->diag_blocks = want_blocks < 2 * sms ? (want_blocks > 0 ? want_blocks : 1) : 2 * sms;
+    B.want(&s->d_diag_part, (size_t)s->diag_blocks * kDiagRows);
+    B.want(&s->d_diag_done, 1);
+    B.want(&s->d_diag, 1);
   }
-  TRY(dalloc(s, &s->d_diag_part, (size_t)s->diag_blocks * kDiagRows));
-  TRY(dalloc(s, &s->d_diag_done, 1));
-  TRY(dalloc(s, &s->d_diag, 1));
+  B.want(&s->d_niac, 2);  // the last pass's; a step's running sums
+  B.want(&s->d_max_nb, 2);
+  B.want(&s->d_itime, 1);
+  void *base = nullptr;
+  TRY(B.commit(&base));
+  s->allocations.push_back(base);
+  TRY(cudaMemset(s->P.rebuild, 1, sizeof(unsigned)));
+  TRY(cudaMemset(G.gen, 0, sizeof(unsigned)));
+  TRY(cudaMemset(G.bar, 0, kGridWords * sizeof(unsigned)));
+  TRY(cudaMemset(words, 0, kWords * sizeof(int)));
+  TRY(cudaMemset(s->d_niac, 0, 2 * sizeof(unsigned long long)));
+  TRY(cudaMemset(s->d_max_nb, 0, 2 * sizeof(int)));
+  G.st.nstream = words;
+  G.st.nhard = words + 1;
+  G.st.recorded = reinterpret_cast<unsigned *>(words + 2);
+  s->d_step_done = reinterpret_cast<unsigned *>(words + 3);
+  s->d_moved = reinterpret_cast<unsigned *>(words + 4);
+  G.st.nlive = words + 5;
+  s->d_ticket = reinterpret_cast<unsigned *>(words + 6);
+  s->d_phases = reinterpret_cast<unsigned *>(words + 8);
+  if (!search_only) {
+    TRY(cudaMemset(mass0, 0, sizeof(double)));
+    s->P.pack_mass0 = mass0;
+    s->W.base = s->d_wall_tab + 3 * nm;
+  }
+  if (s->P.nvrules > 0) {
+    TRY(cudaMemset(V.count, 0, sizeof(int)));
+    TRY(cudaMemset(Gv.bar, 0, kGridWords * sizeof(unsigned)));
+  }
+  TRY(alloc_grid(s));
   TRY(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
   s->own_stream = true;
   {
@@ -948,16 +984,19 @@ extern "C" uph_status uph_sim_create(const uph_params *p, uph_sim **out)
   // non-blocking stream does not wait for
   TRY(cudaDeviceSynchronize());
   TRY(cudaMemsetAsync(s->d_err, 0, sizeof(unsigned), s->stream));
-  TRY(cudaMemsetAsync(s->d_diag_done, 0, sizeof(unsigned), s->stream));
-  TRY(cudaMemsetAsync(s->d_diag, 0, sizeof(DevDiag), s->stream));
+  if (!search_only) {
+    TRY(cudaMemsetAsync(s->d_diag_done, 0, sizeof(unsigned), s->stream));
+    TRY(cudaMemsetAsync(s->d_diag, 0, sizeof(DevDiag), s->stream));
+  }
 #undef TRY
   *out = s;
   return UPH_OK;
 }
 
-namespace {
 void drop_graph(uph_sim *s);
-}
+}  // namespace
+
+extern "C" uph_status uph_sim_create(const uph_params *p, uph_sim **out) { return create_sim(p, out, false); }
 
 extern "C" uph_status uph_sim_destroy(uph_sim *s)
 {
@@ -965,11 +1004,7 @@ extern "C" uph_status uph_sim_destroy(uph_sim *s)
   if (s->stream) cudaStreamSynchronize(s->stream);
   drop_graph(s);
   for (void *p : s->allocations) cudaFree(p);
-  for (void *p : {(void *)s->G.count, (void *)s->G.start, (void *)s->G.fill, (void *)s->G.block_sums,
-                  (void *)s->G.st.slot, (void *)s->G.st.core, (void *)s->G.st.tile, (void *)s->G.st.hard,
-                  (void *)s->G.st.live,
-                  (void *)s->gv.count, (void *)s->gv.start, (void *)s->gv.fill, (void *)s->pe_ip, (void *)s->pe_jp,
-                  (void *)s->pe_r2, (void *)s->pe_w, (void *)s->pe_dw})
+  for (void *p : {s->grid_block, s->stream_block, s->pe_index, s->pe_block, s->pe_kernel})
     if (p) cudaFree(p);
   if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
   for (cudaEvent_t e : s->ev_pool)
@@ -1586,9 +1621,11 @@ extern "C" uph_status uph_sim_pairs(uph_sim *s, int64_t cap, int32_t *i_pair, in
   }
   if (!s->pe_cnt) {
     const int nb = scan_block_sums_needed(nf > 0 ? nf : 1);
-    UPH_CUDA(dalloc(s, &s->pe_cnt, (size_t)nf + 1));
-    UPH_CUDA(dalloc(s, &s->pe_off, (size_t)nf + 1));
-    UPH_CUDA(dalloc(s, &s->pe_bsum, (size_t)nb));
+    Block B;
+    B.want(&s->pe_cnt, (size_t)nf + 1);
+    B.want(&s->pe_off, (size_t)nf + 1);
+    B.want(&s->pe_bsum, (size_t)nb);
+    UPH_CUDA(B.commit(&s->pe_index));
   }
   int *cnt = s->pe_cnt, *off = s->pe_off, *bsum = s->pe_bsum;
   uph_status result = UPH_OK;
@@ -1604,24 +1641,32 @@ extern "C" uph_status uph_sim_pairs(uph_sim *s, int64_t cap, int32_t *i_pair, in
   if (total > cap) {
     result = fail(UPH_NEIGHBOR_OVERFLOW, "pair buffer too small: " + std::to_string(total) + " pairs");
   } else if (total > 0) {
+    // grow by a quarter beyond what is needed, so small growth reallocates
+    // rarely; the kernel values only where they are asked for
+    const int64_t cap2 = (int64_t)total + total / 4 + 1024;
     if (total > s->pe_cap) {
-      // grow by a quarter beyond what is needed, so small growth reallocates rarely
-      UPH_CUDA(cudaStreamSynchronize(q));
-      for (void *p : {(void *)s->pe_ip, (void *)s->pe_jp, (void *)s->pe_r2, (void *)s->pe_w, (void *)s->pe_dw})
-        if (p) cudaFree(p);
-      s->pe_ip = s->pe_jp = nullptr;
-      s->pe_r2 = s->pe_w = s->pe_dw = nullptr;
+      if (s->pe_block) cudaFree(s->pe_block);
+      s->pe_block = nullptr;
       s->pe_cap = 0;
-      const int64_t cap2 = (int64_t)total + total / 4 + 1024;
-      UPH_CUDA(cudaMalloc((void **)&s->pe_ip, sizeof(int32_t) * cap2));
-      UPH_CUDA(cudaMalloc((void **)&s->pe_jp, sizeof(int32_t) * cap2));
-      UPH_CUDA(cudaMalloc((void **)&s->pe_r2, sizeof(double) * cap2));
-      UPH_CUDA(cudaMalloc((void **)&s->pe_w, sizeof(double) * cap2));
-      UPH_CUDA(cudaMalloc((void **)&s->pe_dw, sizeof(double) * 2 * cap2));
+      Block B;
+      B.want(&s->pe_ip, (size_t)cap2);
+      B.want(&s->pe_jp, (size_t)cap2);
+      B.want(&s->pe_r2, (size_t)cap2);
+      UPH_CUDA(B.commit(&s->pe_block));
       s->pe_cap = cap2;
     }
+    if ((w || dwcdx) && total > s->pe_kernel_cap) {
+      if (s->pe_kernel) cudaFree(s->pe_kernel);
+      s->pe_kernel = nullptr;
+      s->pe_kernel_cap = 0;
+      Block B;
+      B.want(&s->pe_w, (size_t)cap2);
+      B.want(&s->pe_dw, 2 * (size_t)cap2);
+      UPH_CUDA(B.commit(&s->pe_kernel));
+      s->pe_kernel_cap = cap2;
+    }
     int32_t *dip = s->pe_ip, *djp = s->pe_jp;
-    double *dr = s->pe_r2, *dww = s->pe_w, *ddw = s->pe_dw;
+    double *dr = s->pe_r2, *dww = w || dwcdx ? s->pe_w : nullptr, *ddw = w || dwcdx ? s->pe_dw : nullptr;
     k_pair_write<<<(nf + 127) / 128, 128, 0, q>>>(s->P, s->S, s->G, off, dip, djp, dr, dww, ddw);
     s->launches++;
     if (i_pair) cudaMemcpyAsync(i_pair, dip, sizeof(int32_t) * total, cudaMemcpyDeviceToHost, q);
@@ -2022,7 +2067,7 @@ extern "C" uph_status uph_search_neighbors(const double *position, int32_t n_flu
   p.domain_hi[0] = hi[0] + pad;
   p.domain_hi[1] = hi[1] + pad;
   uph_sim *s = nullptr;
-  uph_status r = uph_sim_create(&p, &s);
+  uph_status r = create_sim(&p, &s, true);
   if (r != UPH_OK) return r;
   // the reference's own threshold and boundary index, not ones derived from h
   s->P.r2cut = dist;
@@ -2039,7 +2084,6 @@ extern "C" uph_status uph_search_neighbors(const double *position, int32_t n_flu
   if (r == UPH_OK) r = build_cell_list(s);
   // an overcrowded cell (or a position outside the grid) stops here, before
   // any kernel walks the candidates
-  if (r == UPH_OK) r = check_error_word(s);
   if (r == UPH_OK) r = check_error_word(s);
   if (r == UPH_OK) {
     s->have_rates = true;

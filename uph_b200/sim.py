@@ -241,17 +241,28 @@ def search_neighbors(position: np.ndarray, n_fluid: int, particle_boundary: int,
     l = _lib.lib()
     pos = np.ascontiguousarray(position, dtype=np.float64).reshape(-1, 2)
     n = C.c_int64(0)
-    st = l.uph_search_neighbors(pos.ctypes.data, n_fluid, pos.shape[0], particle_boundary, number_of_neighbors,
-                                dist, 0, None, None, None, C.byref(n))
-    if st not in (0, 3):
-        _lib.check(st, "uph_search_neighbors")
+
+    def call(cap, i=None, j=None, r2=None):
+        at = [None if a is None else a.ctypes.data for a in (i, j, r2)]
+        return l.uph_search_neighbors(pos.ctypes.data, n_fluid, pos.shape[0], particle_boundary, number_of_neighbors,
+                                      dist, cap, *at, C.byref(n))
+
+    # room for what a capped search can return at most, where that is a small
+    # multiple of the positions (the pages behind unused room stay untouched);
+    # else a first call that counts
+    cap = n_fluid * min(number_of_neighbors, pos.shape[0])
+    if not 0 < cap <= 1 << 26:
+        st = call(0)
+        if st not in (0, 3):
+            _lib.check(st, "uph_search_neighbors")
+        cap = n.value
+    i = np.empty(cap, np.int32)
+    j = np.empty(cap, np.int32)
+    r2 = np.empty(cap)
+    _lib.check(call(cap, i, j, r2), "uph_search_neighbors")
     k = n.value
-    i = np.zeros(k, np.int32)
-    j = np.zeros(k, np.int32)
-    r2 = np.zeros(k)
-    _lib.check(l.uph_search_neighbors(pos.ctypes.data, n_fluid, pos.shape[0], particle_boundary,
-                                      number_of_neighbors, dist, k, i.ctypes.data, j.ctypes.data, r2.ctypes.data,
-                                      C.byref(n)), "uph_search_neighbors")
+    if k < cap:
+        i, j, r2 = i[:k].copy(), j[:k].copy(), r2[:k].copy()
     return i, j, r2
 
 
