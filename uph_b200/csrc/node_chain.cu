@@ -494,7 +494,9 @@ __global__ void k_swizzle_image(const __nv_bfloat16 *__restrict__ W, int N, int 
 
 }  // namespace
 
-uph_status make_row_tensor_map(CUtensorMap *map, const void *base, int rows, int cols, int row_bytes)
+namespace {
+uph_status encode_map(CUtensorMap *map, CUtensorMapDataType type, int elem, const void *base, int rows, int cols,
+                      int row_bytes, int box_rows)
 {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
@@ -505,17 +507,34 @@ uph_status make_row_tensor_map(CUtensorMap *map, const void *base, int rows, int
       return fail(UPH_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from the driver");
     encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
   }
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (row_bytes & 15) || rows < 1 || cols % 64)
-    return fail(UPH_BAD_ARG, "tensor map: base and row stride must be 16-byte aligned, columns whole boxes");
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (row_bytes & 15) || rows < 1 || cols < 1 || (cols * elem) % 16)
+    return fail(UPH_BAD_ARG, "tensor map: base, row stride and columns must be whole 16-byte words");
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
-  cuuint32_t box[2] = {64, 128};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / elem), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1, 1};
-  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box,
-                            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  const CUresult r = encode(map, type, 2, const_cast<void *>(base), dims, strides, box, estr,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(UPH_CUDA_ERROR, "cuTensorMapEncodeTiled failed");
   return UPH_OK;
+}
+}  // namespace
+
+uph_status make_tensor_map(CUtensorMap *map, const void *base, int rows, int cols, int row_bytes, int box_rows)
+{
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, cols, row_bytes, box_rows);
+}
+
+uph_status make_f32_map(CUtensorMap *map, const void *base, int rows, int cols, int row_bytes)
+{
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, row_bytes, 128);
+}
+
+uph_status make_row_tensor_map(CUtensorMap *map, const void *base, int rows, int cols, int row_bytes)
+{
+  if (cols % 64) return fail(UPH_BAD_ARG, "tensor map: columns must be whole boxes");
+  return make_tensor_map(map, base, rows, cols, row_bytes, 128);
 }
 
 void launch_swizzle_image(const __nv_bfloat16 *W, int N, int K, uint8_t *img, cudaStream_t s)

@@ -40,6 +40,11 @@ struct ChainArgs {
 // `row_bytes`, boxes of 128 rows x 64 columns, 128-byte swizzle (loads and
 // stores of one shared-memory atom).
 uph_status make_row_tensor_map(CUtensorMap *map, const void *base, int rows, int cols, int row_bytes);
+// the same for any number of columns (a multiple of 8) and boxes of box_rows
+// rows x 64 columns; what a box holds beyond the matrix reads as zero
+uph_status make_tensor_map(CUtensorMap *map, const void *base, int rows, int cols, int row_bytes, int box_rows);
+// boxes of 128 rows x 32 FP32 columns, 128-byte swizzle
+uph_status make_f32_map(CUtensorMap *map, const void *base, int rows, int cols, int row_bytes);
 // writes the shared-memory image of W [N x K] (row-major BF16) to img: K/64
 // atoms of N rows x 128 bytes
 void launch_swizzle_image(const __nv_bfloat16 *W, int N, int K, uint8_t *img, cudaStream_t s);

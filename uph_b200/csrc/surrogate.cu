@@ -47,8 +47,7 @@ constexpr int kEdgeThreads = 256;           // 8 warps
 // fixed grid (per-warp partials in a fixed order) of one wave: the edge
 // kernels take 80 registers x 256 threads, so three blocks fit an SM's 64K
 // registers; a fourth block per SM would run as a second, mostly empty wave
-constexpr int kEdgeBlocks = 148 * 3;
-constexpr int kColBlocks = 148 * 2;         // bias-gradient partial sums
+constexpr int kEdgeBlocks = 148 * 3, kEdgeBwdBlocks = 148 * 2;
 constexpr int kSplitMax = 148;              // split-K CTAs of one weight-gradient GEMM tile
 constexpr int kLossBlocks = 148;
 constexpr int kMaxBins = 4096;
@@ -120,15 +119,10 @@ __device__ __forceinline__ void store_bf16x4(bf16 *p, const float v[4])
   *reinterpret_cast<uint2 *>(p) = raw;
 }
 
-// the edge pre-activation, one fixed operation order shared by the forward
-// and backward kernels so both see bit-identical values
-__device__ __forceinline__ float edge_z(float p, float q, const float4 &w, float e0, float e1, float e2, float e3)
-{
-  return __fmaf_rn(w.w, e3, __fmaf_rn(w.z, e2, __fmaf_rn(w.y, e1, __fmaf_rn(w.x, e0, __fadd_rn(p, q)))));
-}
-
 // packed FP32 pairs (sm_100 f32x2 instructions): each half rounds exactly
-// like the scalar FP32 operation, so packed and scalar code agree bitwise
+// like the scalar FP32 operation.  Both edge kernels form a pre-activation as
+// fma(w3, e3, fma(w2, e2, fma(w1, e1, fma(w0, e0, P + Q)))), so both see the
+// same bits.
 typedef unsigned long long f32x2;
 
 __device__ __forceinline__ f32x2 pack2(float lo, float hi)
@@ -257,21 +251,49 @@ __global__ void k_sur_features(int n, const double *__restrict__ u, const double
 }
 
 // ---- edge layer -----------------------------------------------------------------
+// Both edge kernels fetch the next node's edge records (and what else they
+// read of its own) into shared memory by cp.async while they work on a node,
+// its degree having been read a node earlier: without that, a node starts
+// with a chain of three loads.
+__device__ __forceinline__ void cp16(void *dst, const void *src)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp4(void *dst, const void *src)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void cp_wait()
+{
+  asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
+}
+
 // S_i = sum_j relu(P_i + Q_j + W_e e_ij), PQ rows = [P | Q].  A half-warp
 // per node, lane l of the half owning channels [8l, 8l + 8) as four packed
-// FP32 pairs (the operation order of edge_z).  Each warp stages its two
-// nodes' edge records (features + partner) in shared memory, so a partner
-// costs one shared broadcast read and one 16-byte gather of its Q row;
-// partners are summed in graph order.
-__global__ void __launch_bounds__(kEdgeThreads) k_sur_edge_fwd(int n, const bf16 *__restrict__ PQ,
+// FP32 pairs.  A partner costs one shared broadcast read of its record and one
+// 16-byte gather of its Q row; partners are summed in graph order.  Bound by
+// issue and by the gathers' latency at 24 warps per SM: 82 us at 83,000 nodes
+// and 187 at 207,000 (83 and 190 with a node's records fetched when its turn
+// comes; 86 and 203 with the nodes in cell order, which hits L1 no more often).
+__global__ void __launch_bounds__(kEdgeThreads, 3) k_sur_edge_fwd(int n, const bf16 *__restrict__ PQ,
                                                                  const float *__restrict__ we,
                                                                  const int *__restrict__ nbr,
                                                                  const float4 *__restrict__ ef,
                                                                  const int *__restrict__ deg, bf16 *__restrict__ S)
 {
-  __shared__ float4 rec[kEdgeThreads / 32][2][kMaxDeg];
-  __shared__ int recj[kEdgeThreads / 32][2][kMaxDeg];
-  const int lane = threadIdx.x & 31, hl = lane & 15, half = lane >> 4, wib = threadIdx.x >> 5;
+  struct Node {
+    float4 rec[kMaxDeg];
+    uint4 p[16];  // the node's own P row
+    int j[kMaxDeg];
+  };
+  __shared__ Node nodes[2][kEdgeThreads / 16];
+  const int hl = threadIdx.x & 15, hw = threadIdx.x >> 4;
   const int gh = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;  // global half-warp
   const int nh = (gridDim.x * blockDim.x) >> 4;
   const int c0 = hl * 8;
@@ -285,23 +307,32 @@ __global__ void __launch_bounds__(kEdgeThreads) k_sur_edge_fwd(int n, const bf16
     w2[q] = pack2(wa.z, wb.z);
     w3[q] = pack2(wa.w, wb.w);
   }
-  float4 *my = rec[wib][half];
-  int *myj = recj[wib][half];
+  auto fetch = [&](int i, int d, int buf) {
+    Node &N = nodes[buf][hw];
+    if (i < n) {
+      for (int k = hl; k < d; k += 16) {
+        cp16(&N.rec[k], ef + (size_t)i * kMaxDeg + k);
+        cp4(&N.j[k], nbr + (size_t)i * kMaxDeg + k);
+      }
+      cp16(&N.p[hl], PQ + (size_t)i * 2 * kLat + c0);
+    }
+    cp_commit();
+  };
+  auto degree = [&](int i) { return i < n ? deg[i] : 0; };
   const int passes = (n + nh - 1) / nh;  // the same for both halves of a warp
+  int d = degree(gh), d1 = degree(gh + nh);
+  fetch(gh, d, 0);
   for (int ps = 0; ps < passes; ps++) {
     const int i = gh + ps * nh;
-    const bool live = i < n;
-    const int d = live ? deg[i] : 0;
-    __syncwarp();  // the last pass's records are read
-    for (int k = hl; k < d; k += 16) {
-      my[k] = ef[(size_t)i * kMaxDeg + k];
-      myj[k] = nbr[(size_t)i * kMaxDeg + k];
-    }
+    __syncwarp();  // the buffer's last records are read
+    fetch(i + nh, d1, (ps + 1) & 1);
+    const int d2 = degree(i + 2 * nh);
+    cp_wait<1>();
     __syncwarp();
+    const Node &N = nodes[ps & 1][hw];
     f32x2 p[4], acc[4];
     {
-      uint4 praw = make_uint4(0u, 0u, 0u, 0u);
-      if (live) praw = *reinterpret_cast<const uint4 *>(PQ + (size_t)i * 2 * kLat + c0);
+      const uint4 praw = N.p[hl];
       p[0] = bf2_to_f2(praw.x);
       p[1] = bf2_to_f2(praw.y);
       p[2] = bf2_to_f2(praw.z);
@@ -309,37 +340,25 @@ __global__ void __launch_bounds__(kEdgeThreads) k_sur_edge_fwd(int n, const bf16
     }
 #pragma unroll
     for (int q = 0; q < 4; q++) acc[q] = pack2(0.0f, 0.0f);
-    int k = 0;
-    for (; k + 4 <= d; k += 4) {
-      float4 e[4];
-      uint4 qv[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) e[u] = my[k + u];
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        qv[u] = *reinterpret_cast<const uint4 *>(PQ + (size_t)myj[k + u] * 2 * kLat + kLat + c0);
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const f32x2 e0 = pack2(e[u].x, e[u].x), e1 = pack2(e[u].y, e[u].y), e2 = pack2(e[u].z, e[u].z);
-        const f32x2 e3 = pack2(e[u].w, e[u].w);
-        const uint32_t qw[4] = {qv[u].x, qv[u].y, qv[u].z, qv[u].w};
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          acc[q] = add2(acc[q], relu2(fma2(w3[q], e3, fma2(w2[q], e2, fma2(w1[q], e1,
-                                                                              fma2(w0[q], e0, add2(p[q], bf2_to_f2(qw[q]))))))));
-      }
-    }
-    for (; k < d; k++) {
-      const float4 e = my[k];
-      const uint4 qv = *reinterpret_cast<const uint4 *>(PQ + (size_t)myj[k] * 2 * kLat + kLat + c0);
+    auto edge = [&](const float4 &e, const uint4 &qv) {
       const f32x2 e0 = pack2(e.x, e.x), e1 = pack2(e.y, e.y), e2 = pack2(e.z, e.z), e3 = pack2(e.w, e.w);
       const uint32_t qw[4] = {qv.x, qv.y, qv.z, qv.w};
 #pragma unroll
       for (int q = 0; q < 4; q++)
         acc[q] = add2(acc[q], relu2(fma2(w3[q], e3, fma2(w2[q], e2, fma2(w1[q], e1,
                                                                             fma2(w0[q], e0, add2(p[q], bf2_to_f2(qw[q]))))))));
+    };
+    auto q_row = [&](int k) { return *reinterpret_cast<const uint4 *>(PQ + (size_t)N.j[k] * 2 * kLat + kLat + c0); };
+    int k = 0;
+    for (; k + 4 <= d; k += 4) {
+      uint4 qv[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) qv[u] = q_row(k + u);
+#pragma unroll
+      for (int u = 0; u < 4; u++) edge(N.rec[k + u], qv[u]);
     }
-    if (live) {
+    for (; k < d; k++) edge(N.rec[k], q_row(k));
+    if (i < n) {
       float v[8];
 #pragma unroll
       for (int q = 0; q < 4; q++) unpack2(acc[q], v[2 * q], v[2 * q + 1]);
@@ -348,73 +367,144 @@ __global__ void __launch_bounds__(kEdgeThreads) k_sur_edge_fwd(int n, const bf16
       for (int q = 0; q < 4; q++) h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
       *reinterpret_cast<uint4 *>(S + (size_t)i * kLat + c0) = *reinterpret_cast<uint4 *>(&h[0]);
     }
+    d = d1;
+    d1 = d2;
   }
+  cp_wait<0>();
+}
+
+// z > 0 ? v : 0, half by half
+__device__ __forceinline__ f32x2 where_positive(f32x2 z, f32x2 v)
+{
+  float za, zb, va, vb;
+  unpack2(z, za, zb);
+  unpack2(v, va, vb);
+  return pack2(za > 0.0f ? va : 0.0f, zb > 0.0f ? vb : 0.0f);
 }
 
 // gradients of the edge layer, node a as receiver (dP_a, dW_e) and as sender
 // (dQ_a, through every partner b that receives from a: the graph is
-// symmetric and e_ba = (-e_ab.x, -e_ab.y, e_ab.z))
-__global__ void __launch_bounds__(kEdgeThreads) k_sur_edge_bwd(int n, const bf16 *__restrict__ PQ,
-                                                                 const float *__restrict__ we,
-                                                                 const int *__restrict__ nbr,
-                                                                 const float4 *__restrict__ ef,
-                                                                 const int *__restrict__ deg,
-                                                                 const float *__restrict__ dS, bf16 *__restrict__ dPQ,
-                                                                 float *__restrict__ we_part)
+// symmetric and e_ba = (-e_ab.x, -e_ab.y, e_ab.z)).  A warp per node, lane l
+// owning channels [4l, 4l + 4) as two packed FP32 pairs; the rows of four
+// partners (1 KB each: P, Q, dS) are in flight at a time.  Bound by issue and
+// the gathers' latency: 207 us at 83,000 nodes, against 271 with scalar
+// arithmetic under branches and one partner's rows at a time (246 with that and
+// the nodes in cell order).
+__global__ void __launch_bounds__(kEdgeThreads, 2) k_sur_edge_bwd(int n, const bf16 *__restrict__ PQ,
+                                                                   const float *__restrict__ we,
+                                                                   const int *__restrict__ nbr,
+                                                                   const float4 *__restrict__ ef,
+                                                                   const int *__restrict__ deg,
+                                                                   const float *__restrict__ dS,
+                                                                   bf16 *__restrict__ dPQ, float *__restrict__ we_part)
 {
-  const int lane = threadIdx.x & 31;
+  struct Node {
+    float4 rec[kMaxDeg], ds[kMaxDeg];  // the edge records; the node's own dS row
+    uint4 pq[kMaxDeg];                 // its own [P | Q] row
+    int j[kMaxDeg];
+  };
+  __shared__ Node nodes[2][kEdgeThreads / 32];
+  __shared__ float4 red[kEdgeThreads / 32][kLat];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const int c0 = lane * 4;
-  float4 w[4];
-  for (int c = 0; c < 4; c++) w[c] = *reinterpret_cast<const float4 *>(we + (c0 + c) * 4);
-  float g[4][4];
-  for (int c = 0; c < 4; c++) g[c][0] = g[c][1] = g[c][2] = g[c][3] = 0.0f;
-  for (int a = gw; a < n; a += nw) {
-    const int d = deg[a];
-    int myj = 0;
-    float4 mye = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (lane < d) {
-      myj = nbr[(size_t)a * kMaxDeg + lane];
-      mye = ef[(size_t)a * kMaxDeg + lane];
-    }
-    float pa[4], qa[4];
-    load_bf16x4(PQ + (size_t)a * 2 * kLat + c0, pa);
-    load_bf16x4(PQ + (size_t)a * 2 * kLat + kLat + c0, qa);
-    const float4 dsa4 = *reinterpret_cast<const float4 *>(dS + (size_t)a * kLat + c0);
-    const float dsa[4] = {dsa4.x, dsa4.y, dsa4.z, dsa4.w};
-    float dp[4] = {0.f, 0.f, 0.f, 0.f}, dq[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int k = 0; k < d; k++) {
-      const int b = __shfl_sync(0xffffffffu, myj, k);
-      const float e0 = __shfl_sync(0xffffffffu, mye.x, k);
-      const float e1 = __shfl_sync(0xffffffffu, mye.y, k);
-      const float e2 = __shfl_sync(0xffffffffu, mye.z, k);
-      const float e3 = __shfl_sync(0xffffffffu, mye.w, k);
-      float pb[4], qb[4];
-      load_bf16x4(PQ + (size_t)b * 2 * kLat + c0, pb);
-      load_bf16x4(PQ + (size_t)b * 2 * kLat + kLat + c0, qb);
-      const float4 dsb4 = *reinterpret_cast<const float4 *>(dS + (size_t)b * kLat + c0);
-      const float dsb[4] = {dsb4.x, dsb4.y, dsb4.z, dsb4.w};
+  f32x2 w[4][2], g[4][2];
 #pragma unroll
-      for (int c = 0; c < 4; c++) {
-        if (edge_z(pa[c], qb[c], w[c], e0, e1, e2, e3) > 0.0f) {
-          dp[c] += dsa[c];
-          g[c][0] = __fmaf_rn(dsa[c], e0, g[c][0]);
-          g[c][1] = __fmaf_rn(dsa[c], e1, g[c][1]);
-          g[c][2] = __fmaf_rn(dsa[c], e2, g[c][2]);
-          g[c][3] = __fmaf_rn(dsa[c], e3, g[c][3]);
-        }
-        // the reverse edge: dx, dy and the density difference change sign
-        if (edge_z(pb[c], qa[c], w[c], -e0, -e1, e2, -e3) > 0.0f) dq[c] += dsb[c];
-      }
-    }
-    store_bf16x4(dPQ + (size_t)a * 2 * kLat + c0, dp);
-    store_bf16x4(dPQ + (size_t)a * 2 * kLat + kLat + c0, dq);
+  for (int q = 0; q < 2; q++) {
+    const float4 wa = *reinterpret_cast<const float4 *>(we + (c0 + 2 * q) * 4);
+    const float4 wb = *reinterpret_cast<const float4 *>(we + (c0 + 2 * q + 1) * 4);
+    w[0][q] = pack2(wa.x, wb.x);
+    w[1][q] = pack2(wa.y, wb.y);
+    w[2][q] = pack2(wa.z, wb.z);
+    w[3][q] = pack2(wa.w, wb.w);
+    for (int k = 0; k < 4; k++) g[k][q] = pack2(0.0f, 0.0f);
   }
+  auto fetch = [&](int a, int d, int buf) {
+    Node &N = nodes[buf][wib];
+    if (a < n) {
+      if (lane < d) {
+        cp16(&N.rec[lane], ef + (size_t)a * kMaxDeg + lane);
+        cp4(&N.j[lane], nbr + (size_t)a * kMaxDeg + lane);
+      }
+      cp16(&N.ds[lane], dS + (size_t)a * kLat + c0);
+      cp16(&N.pq[lane], PQ + (size_t)a * 2 * kLat + lane * 8);
+    }
+    cp_commit();
+  };
+  auto degree = [&](int a) { return a < n ? deg[a] : 0; };
+  int d = degree(gw), d1 = degree(gw + nw);
+  fetch(gw, d, 0);
+  int turn = 0;
+  for (int a = gw; a < n; a += nw, turn++) {
+    __syncwarp();  // the buffer's last node is done
+    fetch(a + nw, d1, (turn + 1) & 1);
+    const int d2 = degree(a + 2 * nw);
+    cp_wait<1>();
+    __syncwarp();
+    const Node &N = nodes[turn & 1][wib];
+    const uint2 prow = *reinterpret_cast<const uint2 *>(reinterpret_cast<const bf16 *>(N.pq) + c0);
+    const uint2 qrow = *reinterpret_cast<const uint2 *>(reinterpret_cast<const bf16 *>(N.pq) + kLat + c0);
+    const float4 dsa = N.ds[lane];
+    const f32x2 pa[2] = {bf2_to_f2(prow.x), bf2_to_f2(prow.y)}, qa[2] = {bf2_to_f2(qrow.x), bf2_to_f2(qrow.y)};
+    const f32x2 sa[2] = {pack2(dsa.x, dsa.y), pack2(dsa.z, dsa.w)};
+    f32x2 dp[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)}, dq[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
+    auto edge = [&](const float4 &e, const uint2 &pr, const uint2 &qr, const float4 &ds) {
+      const f32x2 e0 = pack2(e.x, e.x), e1 = pack2(e.y, e.y), e2 = pack2(e.z, e.z), e3 = pack2(e.w, e.w);
+      // the reverse edge: dx, dy and the density difference change sign
+      const f32x2 m0 = pack2(-e.x, -e.x), m1 = pack2(-e.y, -e.y), m3 = pack2(-e.w, -e.w);
+      const uint32_t pw[2] = {pr.x, pr.y}, qw[2] = {qr.x, qr.y};
+      const f32x2 sb[2] = {pack2(ds.x, ds.y), pack2(ds.z, ds.w)};
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const f32x2 z = fma2(w[3][q], e3, fma2(w[2][q], e2, fma2(w[1][q], e1, fma2(w[0][q], e0,
+                                                                                 add2(pa[q], bf2_to_f2(qw[q]))))));
+        const f32x2 on = where_positive(z, sa[q]);
+        dp[q] = add2(dp[q], on);
+        g[0][q] = fma2(on, e0, g[0][q]);
+        g[1][q] = fma2(on, e1, g[1][q]);
+        g[2][q] = fma2(on, e2, g[2][q]);
+        g[3][q] = fma2(on, e3, g[3][q]);
+        const f32x2 y = fma2(w[3][q], m3, fma2(w[2][q], e2, fma2(w[1][q], m1, fma2(w[0][q], m0,
+                                                                                 add2(bf2_to_f2(pw[q]), qa[q])))));
+        dq[q] = add2(dq[q], where_positive(y, sb[q]));
+      }
+    };
+    constexpr int kU = 4;
+    for (int k = 0; k < d; k += kU) {
+      uint2 pr[kU], qr[kU];
+      float4 ds[kU];
+#pragma unroll
+      for (int u = 0; u < kU; u++) {
+        const int b = N.j[min(k + u, d - 1)];
+        const bf16 *row = PQ + (size_t)b * 2 * kLat + c0;
+        pr[u] = *reinterpret_cast<const uint2 *>(row);
+        qr[u] = *reinterpret_cast<const uint2 *>(row + kLat);
+        ds[u] = *reinterpret_cast<const float4 *>(dS + (size_t)b * kLat + c0);
+      }
+#pragma unroll
+      for (int u = 0; u < kU; u++)
+        if (k + u < d) edge(N.rec[k + u], pr[u], qr[u], ds[u]);
+    }
+    float v[4];
+    unpack2(dp[0], v[0], v[1]);
+    unpack2(dp[1], v[2], v[3]);
+    store_bf16x4(dPQ + (size_t)a * 2 * kLat + c0, v);
+    unpack2(dq[0], v[0], v[1]);
+    unpack2(dq[1], v[2], v[3]);
+    store_bf16x4(dPQ + (size_t)a * 2 * kLat + kLat + c0, v);
+    d = d1;
+    d1 = d2;
+  }
+  cp_wait<0>();
   // the block's 8 warps summed in warp order: one partial row per block
-  __shared__ float4 red[kEdgeThreads / 32][kLat];
-  const int wib = threadIdx.x >> 5;
-  for (int c = 0; c < 4; c++) red[wib][c0 + c] = make_float4(g[c][0], g[c][1], g[c][2], g[c][3]);
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    float lo[4], hi[4];
+    for (int k = 0; k < 4; k++) unpack2(g[k][q], lo[k], hi[k]);
+    red[wib][c0 + 2 * q] = make_float4(lo[0], lo[1], lo[2], lo[3]);
+    red[wib][c0 + 2 * q + 1] = make_float4(hi[0], hi[1], hi[2], hi[3]);
+  }
   __syncthreads();
   if (threadIdx.x < kLat) {
     float4 t = red[0][threadIdx.x];
@@ -454,16 +544,14 @@ inline void sum_rows(const float *part, int rows, int cols, float *out, cudaStre
   k_sum_rows<<<(cols + 31) / 32, 1024, 0, s>>>(part, rows, cols, out);
 }
 
-// column sums of a BF16 [n x cols] block (ld >= cols): per-block partials
-__global__ void k_colsum_part(const bf16 *__restrict__ src, int ld, int cols, int n, int rows_per_block,
-                              float *__restrict__ part)
+// column sums of a BF16 [n x cols] block (ld >= cols), few rows
+__global__ void k_colsum(const bf16 *__restrict__ src, int ld, int cols, int n, float *__restrict__ out)
 {
-  const int c = threadIdx.x;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;
-  const int r0 = blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
   float s = 0.0f;
-  for (int r = r0; r < r1; r++) s += __bfloat162float(src[(size_t)r * ld + c]);
-  part[(size_t)blockIdx.x * cols + c] = s;
+  for (int r = 0; r < n; r++) s += __bfloat162float(src[(size_t)r * ld + c]);
+  out[c] = s;
 }
 
 // mean squared error over the fluid rows' 5 outputs; dO = dL/dout in BF16
@@ -832,6 +920,12 @@ uph_status prepare(uph_surrogate *s, const NodesView &nv)
   return UPH_OK;
 }
 
+#define TRYS(x)                     \
+  do {                              \
+    uph_status r_ = (x);            \
+    if (r_ != UPH_OK) return r_;    \
+  } while (0)
+
 struct Gemm {
   GemmCall c;
   Gemm(const void *A, int lda, const void *B, int ldb, int M, int N, int K)
@@ -852,8 +946,10 @@ uph_status run(uph_surrogate *s, GemmCall c)
   return launch_tc_gemm(c, s->stream);
 }
 
-// weight gradient dW[M x N] = sum over nodes of dY[node][M-index] X[node][N-index]
-uph_status wgrad(uph_surrogate *s, const bf16 *dY, int ldy, int M, const bf16 *X, int ldx, int N, int n, float *dst)
+// weight gradient dW[M x N] = sum over nodes of dY[node][M-index] X[node][N-index],
+// and the bias gradient db[M], the column sums of dY (db may be null)
+uph_status wgrad(uph_surrogate *s, const bf16 *dY, int ldy, int M, const bf16 *X, int ldx, int N, int n, float *dst,
+                 float *db)
 {
   GemmCall c;
   c.A = dY;
@@ -871,22 +967,16 @@ uph_status wgrad(uph_surrogate *s, const bf16 *dY, int ldy, int M, const bf16 *X
   c.partials = s->partials;
   c.c_f32 = dst;
   c.ldc = N;
-  return run(s, c);
-}
-
-uph_status colsum(uph_surrogate *s, const bf16 *src, int ld, int cols, int n, float *dst)
-{
-  const int rpb = (n + kColBlocks - 1) / kColBlocks;
-  k_colsum_part<<<kColBlocks, cols, 0, s->stream>>>(src, ld, cols, n, rpb, s->colpart);
-  sum_rows(s->colpart, kColBlocks, cols, dst, s->stream);
+  if (db && c.splits > 1) {
+    c.col_sums = db;
+    c.col_partials = s->colpart;
+  }
+  TRYS(run(s, c));
+  if (db && c.splits == 1) {  // at most 64 nodes
+    k_colsum<<<(M + 127) / 128, 128, 0, s->stream>>>(dY, ldy, M, n, db);
+  }
   return UPH_OK;
 }
-
-#define TRYS(x)                     \
-  do {                              \
-    uph_status r_ = (x);            \
-    if (r_ != UPH_OK) return r_;    \
-  } while (0)
 
 uph_status forward_net(uph_surrogate *s, int n)
 {
@@ -1052,8 +1142,7 @@ uph_status backward_net(uph_surrogate *s, int n)
   const int rounds = s->cfg.rounds;
   UPH_CUDA(cudaMemsetAsync(G, 0, sizeof(float) * o.total, q));
   // decoder
-  TRYS(wgrad(s, s->dO, kOutPad, kOutPad, s->d1, kLat, kLat, n, G + o.dec2_w));
-  TRYS(colsum(s, s->dO, kOutPad, kOutPad, n, G + o.dec2_b));
+  TRYS(wgrad(s, s->dO, kOutPad, kOutPad, s->d1, kLat, kLat, n, G + o.dec2_w, G + o.dec2_b));
   {
     GemmCall c;  // dz = (dO . Dec2) masked by d1 > 0
     c.A = s->dO; c.lda = kOutPad; c.B = Wb + o.dec2_w; c.ldb = kLat; c.b_trans = 1;
@@ -1061,21 +1150,17 @@ uph_status backward_net(uph_surrogate *s, int n)
     c.mask = s->d1; c.ldm = kLat; c.c_bf16 = s->dz; c.ldc = kLat;
     TRYS(run(s, c));
   }
-  TRYS(wgrad(s, s->dz, kLat, kLat, s->cat[rounds], 2 * kLat, kLat, n, G + o.dec1_w));
-  TRYS(colsum(s, s->dz, kLat, kLat, n, G + o.dec1_b));
+  TRYS(wgrad(s, s->dz, kLat, kLat, s->cat[rounds], 2 * kLat, kLat, n, G + o.dec1_w, G + o.dec1_b));
   {
     GemmCall c;  // dh = dz . Dec1
     c.A = s->dz; c.lda = kLat; c.B = Wb + o.dec1_w; c.ldb = kLat; c.b_trans = 1;
     c.M = n; c.N = kLat; c.K = kLat;
-    c.c_f32 = s->dh; c.ldc = kLat;
+    c.c_f32 = s->dh; c.c_bf16 = s->dhb; c.ldc = kLat;
     TRYS(run(s, c));
   }
-  const size_t nl = (size_t)n * kLat;
   for (int r = rounds - 1; r >= 0; r--) {
     const RoundOff &ro = o.r[r];
-    k_f32_to_bf16<<<(unsigned)((nl + 255) / 256), 256, 0, q>>>(s->dh, s->dhb, nl);
-    TRYS(wgrad(s, s->dhb, kLat, kLat, s->u[r], kLat, kLat, n, G + ro.n2_w));
-    TRYS(colsum(s, s->dhb, kLat, kLat, n, G + ro.n2_b));
+    TRYS(wgrad(s, s->dhb, kLat, kLat, s->u[r], kLat, kLat, n, G + ro.n2_w, G + ro.n2_b));
     {
       GemmCall c;  // dz = (dh . N2) masked by u > 0
       c.A = s->dhb; c.lda = kLat; c.B = Wb + ro.n2_w; c.ldb = kLat; c.b_trans = 1;
@@ -1083,8 +1168,7 @@ uph_status backward_net(uph_surrogate *s, int n)
       c.mask = s->u[r]; c.ldm = kLat; c.c_bf16 = s->dz; c.ldc = kLat;
       TRYS(run(s, c));
     }
-    TRYS(wgrad(s, s->dz, kLat, kLat, s->cat[r], 2 * kLat, 2 * kLat, n, G + ro.n1_w));
-    TRYS(colsum(s, s->dz, kLat, kLat, n, G + ro.n1_b));
+    TRYS(wgrad(s, s->dz, kLat, kLat, s->cat[r], 2 * kLat, 2 * kLat, n, G + ro.n1_w, G + ro.n1_b));
     {
       GemmCall c;  // dh += dz . N1[:, :128]
       c.A = s->dz; c.lda = kLat; c.B = Wb + ro.n1_w; c.ldb = 2 * kLat; c.b_trans = 1;
@@ -1099,7 +1183,7 @@ uph_status backward_net(uph_surrogate *s, int n)
       c.c_bf16 = s->dm; c.ldc = kLat;
       TRYS(run(s, c));
     }
-    TRYS(wgrad(s, s->dm, kLat, kLat, s->S[r], kLat, kLat, n, G + ro.w2));
+    TRYS(wgrad(s, s->dm, kLat, kLat, s->S[r], kLat, kLat, n, G + ro.w2, nullptr));
     {
       GemmCall c;  // dS = dm . W2
       c.A = s->dm; c.lda = kLat; c.B = Wb + ro.w2; c.ldb = kLat; c.b_trans = 1;
@@ -1107,22 +1191,19 @@ uph_status backward_net(uph_surrogate *s, int n)
       c.c_f32 = s->dS; c.ldc = kLat;
       TRYS(run(s, c));
     }
-    k_sur_edge_bwd<<<kEdgeBlocks, kEdgeThreads, 0, q>>>(n, s->PQ[r], s->w + ro.we, s->nbr, s->ef, s->deg, s->dS,
+    k_sur_edge_bwd<<<kEdgeBwdBlocks, kEdgeThreads, 0, q>>>(n, s->PQ[r], s->w + ro.we, s->nbr, s->ef, s->deg, s->dS,
                                                         s->dPQ, s->wepart);
-    sum_rows(s->wepart, kEdgeBlocks, kLat * 4, G + ro.we, q);
-    TRYS(wgrad(s, s->dPQ, 2 * kLat, 2 * kLat, s->cat[r], 2 * kLat, kLat, n, G + ro.pq_w));
-    TRYS(colsum(s, s->dPQ, 2 * kLat, 2 * kLat, n, G + ro.pq_b));
+    sum_rows(s->wepart, kEdgeBwdBlocks, kLat * 4, G + ro.we, q);
+    TRYS(wgrad(s, s->dPQ, 2 * kLat, 2 * kLat, s->cat[r], 2 * kLat, kLat, n, G + ro.pq_w, G + ro.pq_b));
     {
-      GemmCall c;  // dh += dPQ . W_pq
+      GemmCall c;  // dh += dPQ . W_pq, and its BF16 copy for the next round down
       c.A = s->dPQ; c.lda = 2 * kLat; c.B = Wb + ro.pq_w; c.ldb = kLat; c.b_trans = 1;
       c.M = n; c.N = kLat; c.K = 2 * kLat;
-      c.accumulate = 1; c.c_f32 = s->dh; c.ldc = kLat;
+      c.accumulate = 1; c.c_f32 = s->dh; c.c_bf16 = s->dhb; c.ldc = kLat;
       TRYS(run(s, c));
     }
   }
-  k_f32_to_bf16<<<(unsigned)((nl + 255) / 256), 256, 0, q>>>(s->dh, s->dhb, nl);
-  TRYS(wgrad(s, s->dhb, kLat, kLat, s->a1, kLat, kLat, n, G + o.enc2_w));
-  TRYS(colsum(s, s->dhb, kLat, kLat, n, G + o.enc2_b));
+  TRYS(wgrad(s, s->dhb, kLat, kLat, s->a1, kLat, kLat, n, G + o.enc2_w, G + o.enc2_b));
   {
     GemmCall c;  // dz = (dh . Enc2) masked by a1 > 0
     c.A = s->dhb; c.lda = kLat; c.B = Wb + o.enc2_w; c.ldb = kLat; c.b_trans = 1;
@@ -1130,8 +1211,7 @@ uph_status backward_net(uph_surrogate *s, int n)
     c.mask = s->a1; c.ldm = kLat; c.c_bf16 = s->dz; c.ldc = kLat;
     TRYS(run(s, c));
   }
-  TRYS(wgrad(s, s->dz, kLat, kLat, s->F, kFeat, kFeat, n, G + o.enc1_w));
-  TRYS(colsum(s, s->dz, kLat, kLat, n, G + o.enc1_b));
+  TRYS(wgrad(s, s->dz, kLat, kLat, s->F, kFeat, kFeat, n, G + o.enc1_w, G + o.enc1_b));
   UPH_CUDA(cudaGetLastError());
   return UPH_OK;
 }
@@ -1219,7 +1299,7 @@ extern "C" uph_status uph_sur_create(const uph_sur_config *cfg, int32_t node_cap
   A(&s->dh, c * kLat);
   A(&s->dS, c * kLat);
   A(&s->partials, (size_t)kSplitMax * 128 * 128);
-  A(&s->colpart, (size_t)kColBlocks * 2 * kLat);
+  A(&s->colpart, (size_t)kSplitMax * 2 * kLat);
   A(&s->wepart, (size_t)kEdgeBlocks * kLat * 4);
   A(&s->losspart, kLossBlocks);
   A(&s->lossval, 1);

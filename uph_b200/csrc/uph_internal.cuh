@@ -380,6 +380,9 @@ struct GemmCall {
   int ldc16 = 0;  // leading dimension of c_bf16 (0: ldc)
   int splits = 1;
   float *partials = nullptr;
+  // split-K with a transposed A: col_sums[M] = the sums of A's columns over
+  // K, through col_partials (splits * M floats)
+  float *col_sums = nullptr, *col_partials = nullptr;
   unsigned *err = nullptr;
   int stall = 0;  // self-test: each CTA first waits on a barrier nothing arrives at
 };
