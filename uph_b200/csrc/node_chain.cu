@@ -12,18 +12,27 @@
 //
 // Two persistent CTAs per SM, 96 KiB of shared memory each:
 //   X  2 atoms   the tile's first operand (F or S), then m, u, ... and P
-//   H  2 atoms   h, updated in place by the residual layer
-//   W  2 atoms   one weight piece (and Q while [P | Q] is stored)
+//   H  2 atoms   h, updated in place by the residual layer, at last Q
+//   W  2 atoms   one weight piece
 // (an atom = 128 rows x 64 BF16 columns in the 128-byte-swizzled K-major
 // layout of the UMMA descriptors).  Inputs arrive by TMA (2-D tensor maps
 // with 128-byte swizzle, no multicast), weight pieces as pre-swizzled images
-// by bulk copies, all completing on mbarriers.  One thread issues each
-// piece's MMAs into the CTA's 256-column TMEM accumulator; after a layer's
-// last piece the four warps read their 32 TMEM lanes (one row per thread),
-// apply bias / residual / ReLU and write BF16 into shared memory; h and
-// [P | Q] leave the SM as TMA tensor stores of those swizzled atoms.  One
-// CTA's chain is serial (MMA -> epilogue -> next MMA); the other CTA on the
-// SM fills its waits.
+// by bulk copies, all completing on mbarriers; h and [P | Q] leave the SM as
+// TMA tensor stores of swizzled atoms.
+//
+// One thread of a ninth warp produces: it fetches, issues every piece's MMAs,
+// refills the weight slot as soon as a piece is done, and stores.  Eight warps
+// run the epilogues (TMEM lane = row, a warp takes 64 of a layer's 128 columns):
+// bias, residual, ReLU, BF16 into shared memory.  Layers alternate between the
+// two 128-column halves of the CTA's TMEM, so a piece that needs nothing of
+// the running epilogue (N1's h half, W_Q, the next tile's first) is multiplied
+// beside it.
+//
+// Bound by the chain of a tile (MMA, epilogue, next MMA), which the SM's two
+// CTAs overlap, and by one weight piece's way from L2 per MMA; the tensor pipe
+// is busy for some 20 us of a round at 207,000 nodes.  A round there: NEWR us
+// (encoder NEWE, last round NEWL), against 114 (90, 91) with four warps that
+// waited for every load, MMA and store in turn.
 //
 // The arithmetic is that of the unfused path (tc_gemm.cu) step for step --
 // the same K order of MMAs, FP32 bias then residual, the same BF16 rounding
@@ -48,48 +57,75 @@ constexpr int kOffH = 2 * kAtom;       // 2 atoms: h
 constexpr int kOffW = 4 * kAtom;       // 2 atoms: one weight piece (128 x 128)
 constexpr int kSmemUsed = 6 * kAtom;   // 96 KiB: two CTAs per SM
 constexpr int kSmemBytes = kSmemUsed + 1024;
-constexpr int kThreads = 128;
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = 32 * (kEpiWarps + 1);
+constexpr int kMaxLayers = 5;
 constexpr int kPieceBytes = 2 * kAtom;
 constexpr long long kWaitLimit = 1LL << 26;
 
 enum Buf : int { BUF_X = 0, BUF_H = 1 };
 
-// what the epilogue after a layer's last piece does with the accumulator
+// what a layer's epilogue does with its accumulator
 enum Epi : int {
-  EPI_NONE = 0,      // not the layer's last piece
-  EPI_X = 1,         // (+ bias) (ReLU) -> BF16 into X
-  EPI_H = 2,         // + bias -> BF16 into H (the encoder's h0)
-  EPI_RESIDUAL = 3,  // + bias + h -> BF16 into H
-  EPI_PQ = 4,        // 256 columns + bias -> BF16, P staged in X and Q in the weight slot, stored by TMA
-  EPI_OUT = 5,       // columns 0..15 + bias -> FP32 to out
+  EPI_X = 0,         // (+ bias) (ReLU) -> BF16 into X
+  EPI_H = 1,         // + bias -> BF16 into H (the encoder's h0; Q)
+  EPI_RESIDUAL = 2,  // + bias + h -> BF16 into H
+  EPI_OUT = 3,       // columns 0..15 + bias -> FP32 to out
 };
 
-struct PieceSpec {
-  int a;     // A operand buffer
-  int col;   // TMEM column of the accumulator
-  int acc;   // accumulate onto it
-  int epi;   // EPI_NONE for all but a layer's last piece
+struct LayerSpec {
+  int epi;
   int relu;
 };
 
-__host__ __device__ inline int piece_count(int mode) { return mode == CHAIN_ENCODER ? 4 : 6; }
+struct PieceSpec {
+  int a;      // A operand buffer
+  int first;  // starts its layer's accumulator
+  int last;   // completes it
+  int after;  // reads what the layer before left in shared memory
+};
 
-// encoder: E1 | E2 | W_P W_Q;  round: W2 | N1a N1b | N2 | W_P W_Q;
+__host__ __device__ inline int piece_count(int mode) { return mode == CHAIN_ENCODER ? 4 : 6; }
+__host__ __device__ inline int layer_count(int mode) { return mode == CHAIN_ENCODER ? 4 : 5; }
+
+// encoder: E1 | E2 | W_P | W_Q;  round: W2 | N1a N1b | N2 | W_P | W_Q;
 // last round: W2 | N1a N1b | N2 | Dec1 | Dec2
 __device__ __forceinline__ PieceSpec piece_of(int mode, int p)
 {
   if (mode == CHAIN_ENCODER) {
-    if (p == 0) return PieceSpec{BUF_X, 0, 0, EPI_X, 1};
-    if (p == 1) return PieceSpec{BUF_X, 0, 0, EPI_H, 0};
-    if (p == 2) return PieceSpec{BUF_H, 0, 0, EPI_NONE, 0};
-    return PieceSpec{BUF_H, 128, 0, EPI_PQ, 0};
+    if (p == 0) return PieceSpec{BUF_X, 1, 1, 0};
+    if (p == 1) return PieceSpec{BUF_X, 1, 1, 1};
+    if (p == 2) return PieceSpec{BUF_H, 1, 1, 1};
+    return PieceSpec{BUF_H, 1, 1, 0};
   }
-  if (p == 0) return PieceSpec{BUF_X, 0, 0, EPI_X, 0};
-  if (p == 1) return PieceSpec{BUF_H, 0, 0, EPI_NONE, 0};
-  if (p == 2) return PieceSpec{BUF_X, 0, 1, EPI_X, 1};
-  if (p == 3) return PieceSpec{BUF_X, 0, 0, EPI_RESIDUAL, 0};
-  if (mode == CHAIN_ROUND) return p == 4 ? PieceSpec{BUF_H, 0, 0, EPI_NONE, 0} : PieceSpec{BUF_H, 128, 0, EPI_PQ, 0};
-  return p == 4 ? PieceSpec{BUF_H, 0, 0, EPI_X, 1} : PieceSpec{BUF_X, 0, 0, EPI_OUT, 0};
+  if (p == 0) return PieceSpec{BUF_X, 1, 1, 0};
+  if (p == 1) return PieceSpec{BUF_H, 1, 0, 0};
+  if (p == 2) return PieceSpec{BUF_X, 0, 1, 1};
+  if (p == 3) return PieceSpec{BUF_X, 1, 1, 1};
+  if (p == 4) return PieceSpec{BUF_H, 1, 1, 1};
+  return mode == CHAIN_ROUND ? PieceSpec{BUF_H, 1, 1, 0} : PieceSpec{BUF_X, 1, 1, 1};
+}
+
+__device__ __forceinline__ LayerSpec layer_of(int mode, int l)
+{
+  if (mode == CHAIN_ENCODER) {
+    if (l == 0) return LayerSpec{EPI_X, 1};
+    return l == 2 ? LayerSpec{EPI_X, 0} : LayerSpec{EPI_H, 0};
+  }
+  if (l == 0) return LayerSpec{EPI_X, 0};
+  if (l == 1) return LayerSpec{EPI_X, 1};
+  if (l == 2) return LayerSpec{EPI_RESIDUAL, 0};
+  if (mode == CHAIN_ROUND) return l == 3 ? LayerSpec{EPI_X, 0} : LayerSpec{EPI_H, 0};
+  return l == 3 ? LayerSpec{EPI_X, 1} : LayerSpec{EPI_OUT, 0};
+}
+
+// a layer's bias: that of its last piece, W_P and W_Q sharing W_Q's 256 values
+__device__ __forceinline__ const float *bias_of(const ChainArgs &a, int l)
+{
+  const int np = piece_count(a.mode);
+  if (a.mode != CHAIN_LAST && l == layer_count(a.mode) - 2) return a.piece[np - 1].bias;
+  if (a.mode != CHAIN_LAST && l == layer_count(a.mode) - 1) return a.piece[np - 1].bias + 128;
+  return a.piece[a.mode == CHAIN_ENCODER || l == 0 ? l : l + 1].bias;
 }
 
 __device__ __forceinline__ uint32_t su32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -237,247 +273,252 @@ __device__ __forceinline__ void issue_piece(uint32_t tmem, uint32_t a, uint32_t 
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+{
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+struct ChainBars {
+  uint64_t x, h, w;    // the tile's first operand, h and the weight piece have arrived
+  uint64_t part;       // an MMA that does not complete its layer is done
+  uint64_t layer[2];   // the MMAs of layer number g (counted over the tiles) are done: [g % 2]
+  uint64_t epi[2];     // its epilogue is done: [g % 2], one arrival per warp
+};
+
 __global__ void __launch_bounds__(kThreads, 2) k_node_chain(const __grid_constant__ ChainArgs a)
 {
   extern __shared__ uint8_t smem_raw[];
-  // X tile, h tile, weight piece, intermediate MMA, final MMA
-  __shared__ uint64_t bars[5];
+  __shared__ ChainBars bars;
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_abort;
   __shared__ int s_mma_pending;  // set by the final drain: an MMA never completed
-  __shared__ float s_bias[256];  // the current layer's bias
+  __shared__ float s_bias[kMaxLayers][128];
   uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sb = su32(sm);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int r = warp * 32 + lane;  // tile row = TMEM lane of this thread
-  const int NP = piece_count(a.mode);
-  const bool has_h = a.mode != CHAIN_ENCODER;
+  const int NP = piece_count(a.mode), NL = layer_count(a.mode);
+  const int stride = gridDim.x, first_tile = blockIdx.x;
+  auto tile_of = [&](int it) { return first_tile + it * stride; };
 
-  if (warp == 0) {
+  if (warp == kEpiWarps) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&tmem_slot)), "r"(256));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
   if (tid == 0) {
-    for (int b = 0; b < 5; b++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&bars[b])));
+    auto init = [](uint64_t *b, int count) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(b)), "r"(count));
+    };
+    init(&bars.x, 1);
+    init(&bars.h, 1);
+    init(&bars.w, 1);
+    init(&bars.part, 1);
+    for (int k = 0; k < 2; k++) {
+      init(&bars.layer[k], 1);
+      init(&bars.epi[k], kEpiWarps);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    s_abort = 0;
     s_mma_pending = 0;
+  }
+  for (int l = 0; l < NL; l++) {
+    const float *bias = bias_of(a, l);
+    const int ncol = layer_of(a.mode, l).epi == EPI_OUT ? 16 : 128;
+    if (bias && tid < ncol) s_bias[l][tid] = bias[tid];
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  const uint32_t bar_x = su32(&bars[0]), bar_h = su32(&bars[1]), bar_w = su32(&bars[2]);
-  const uint32_t bar_mi = su32(&bars[3]), bar_m = su32(&bars[4]);
-  const uint32_t idesc = static_cast<uint32_t>(
-      cute::UMMA::make_instr_desc<cute::bfloat16_t, cute::bfloat16_t, float, 128, 128, cute::UMMA::Major::K,
-                                  cute::UMMA::Major::K>());
 
-  // barrier phases: every thread waits on bar_m (and on bar_h before the
-  // residual); thread 0 also on the inputs, the weights and bar_mi
-  uint32_t ph_m = 0, ph_h_all = 0, ph_x = 0, ph_h = 0, ph_w = 0, ph_mi = 0;
-  bool pend_x = false, pend_h = false, pend_w = false, pend_mi = false, pend_m = false;
-  const int stride = gridDim.x;
-  const int first_tile = blockIdx.x;
-  auto tile_of = [&](int it) { return first_tile + it * stride; };
-  auto fail_wait = [&]() {
-    s_abort = 1;
-    atomicOr(a.err, ERR_TIMEOUT);
-  };
-  // thread 0; a wait that gave up leaves the phase pending, so the final
-  // drain waits for that same phase again
-  auto wait0 = [&](uint32_t bar, uint32_t &ph, bool &pend) {
-    const bool ok = mbar_wait(bar, ph);
-    if (ok) {
-      ph ^= 1u;
-      pend = false;
-    }
-    return ok;
-  };
-  // thread 0: piece g (piece g % NP of iteration g / NP) into the weight slot
-  auto issue_weight = [&](int g) {
-    if (tile_of(g / NP) >= a.ntiles) return;
-    mbar_expect(bar_w, kPieceBytes);
-    bulk_load(sb + kOffW, a.piece[g % NP].img, kAtom, bar_w);
-    bulk_load(sb + kOffW + kAtom, a.piece[g % NP].img + kAtom, kAtom, bar_w);
-    pend_w = true;
-  };
-  auto issue_x = [&](int tile) {
-    mbar_expect(bar_x, 2 * kAtom);
-    tma_load_box(sb + kOffX, &a.tm_a, 0, tile * 128, bar_x);
-    tma_load_box(sb + kOffX + kAtom, &a.tm_a, 64, tile * 128, bar_x);
-    pend_x = true;
-  };
-  auto issue_h = [&](int tile) {
-    mbar_expect(bar_h, 2 * kAtom);
-    tma_load_box(sb + kOffH, &a.tm_h, 0, tile * 128, bar_h);
-    tma_load_box(sb + kOffH + kAtom, &a.tm_h, 64, tile * 128, bar_h);
-    pend_h = true;
-  };
-
-  if (tid == 0 && first_tile < a.ntiles) {
-    issue_weight(0);
-    issue_x(first_tile);
-    if (has_h) issue_h(first_tile);
-  }
-
-  bool stop = false;
-  for (int it = 0; !stop && tile_of(it) < a.ntiles; it++) {
-    const int row0 = tile_of(it) * 128;
-    const bool next = tile_of(it + 1) < a.ntiles;
-    for (int p = 0; p < NP && !stop; p++) {
-      const PieceSpec ps = piece_of(a.mode, p);
-      const int g = it * NP + p;
-      // producer: weights (and this tile's inputs on first use), then the MMA
-      if (tid == 0) {
-        bool ok = wait0(bar_w, ph_w, pend_w);
-        if (ok && p == 0) ok = wait0(bar_x, ph_x, pend_x);
-        if (ok && p == 1 && has_h) ok = wait0(bar_h, ph_h, pend_h);
+  if (warp == kEpiWarps) {
+    if (lane == 0) {
+      const uint32_t bar_x = su32(&bars.x), bar_h = su32(&bars.h), bar_w = su32(&bars.w), bar_part = su32(&bars.part);
+      const uint32_t idesc = static_cast<uint32_t>(
+          cute::UMMA::make_instr_desc<cute::bfloat16_t, cute::bfloat16_t, float, 128, 128, cute::UMMA::Major::K,
+                                      cute::UMMA::Major::K>());
+      // barrier phases; a wait that gave up leaves its phase pending, and the
+      // drain below waits for that same phase again
+      uint32_t ph_x = 0, ph_h = 0, ph_w = 0, ph_part = 0;
+      bool pend_x = false, pend_h = false, pend_w = false, pend_part = false, pend_layer = false;
+      auto wait_on = [&](uint32_t bar, uint32_t &ph, bool &pend) {
+        const bool ok = mbar_wait(bar, ph);
         if (ok) {
+          ph ^= 1u;
+          pend = false;
+        }
+        return ok;
+      };
+      int g = 0;     // the layer at work, counted over the tiles
+      int done = 0;  // epilogues seen done
+      auto wait_epilogues = [&](int count) {
+        bool ok = true;
+        while (ok && done < count) {
+          ok = mbar_wait(su32(&bars.epi[done & 1]), (done >> 1) & 1);
+          if (ok) done++;
+        }
+        return ok;
+      };
+      // piece q % NP of iteration q / NP into the weight slot
+      auto issue_weight = [&](int q) {
+        if (tile_of(q / NP) >= a.ntiles) return;
+        mbar_expect(bar_w, kPieceBytes);
+        bulk_load(sb + kOffW, a.piece[q % NP].img, kAtom, bar_w);
+        bulk_load(sb + kOffW + kAtom, a.piece[q % NP].img + kAtom, kAtom, bar_w);
+        pend_w = true;
+      };
+      auto issue_x = [&](int tile) {
+        if (tile >= a.ntiles) return;
+        mbar_expect(bar_x, 2 * kAtom);
+        tma_load_box(sb + kOffX, &a.tm_a, 0, tile * 128, bar_x);
+        tma_load_box(sb + kOffX + kAtom, &a.tm_a, 64, tile * 128, bar_x);
+        pend_x = true;
+      };
+      auto issue_h = [&](int tile) {
+        if (tile >= a.ntiles || a.mode == CHAIN_ENCODER) return;
+        mbar_expect(bar_h, 2 * kAtom);
+        tma_load_box(sb + kOffH, &a.tm_h, 0, tile * 128, bar_h);
+        tma_load_box(sb + kOffH + kAtom, &a.tm_h, 64, tile * 128, bar_h);
+        pend_h = true;
+      };
+      auto store = [&](const CUtensorMap *map, int off, int x, int row) {
+        tma_store_box(map, sb + off, x, row);
+        tma_store_box(map, sb + off + kAtom, x + 64, row);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      };
+      // the stores so far have read shared memory
+      auto stores_read = [] { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); };
+
+      issue_weight(0);
+      issue_x(first_tile);
+      issue_h(first_tile);
+      const bool pq = a.mode != CHAIN_LAST;  // the chain ends in [P | Q]
+      const int h_piece = NP - 2;            // the first to read the finished h
+      bool ok = true;
+      for (int it = 0; ok && tile_of(it) < a.ntiles; it++) {
+        const int row0 = tile_of(it) * 128;
+        for (int p = 0; p < NP; p++) {
+          const PieceSpec ps = piece_of(a.mode, p);
+          ok = wait_on(bar_w, ph_w, pend_w);
+          if (ok && p == 0) ok = wait_on(bar_x, ph_x, pend_x);
+          if (ok && p == 1 && a.mode != CHAIN_ENCODER) ok = wait_on(bar_h, ph_h, pend_h);
+          // the operand is the last layer's result, or else the accumulator
+          // is that of the layer before it
+          if (ok) ok = wait_epilogues(ps.after ? g : g - 1);
+          if (!ok) break;
+          if (p == h_piece && a.store_h) store(&a.tm_hout, kOffH, 0, row0);
+          if (p == NP - 1 && pq) stores_read();  // Q will overwrite h
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          issue_piece(tmem + ps.col, sb + (ps.a == BUF_X ? kOffX : kOffH), sb + kOffW, idesc, ps.acc,
-                      ps.epi == EPI_NONE ? bar_mi : bar_m);
-          if (ps.epi == EPI_NONE) {
-            pend_mi = true;
-            // the next piece of this layer needs the slot: wait for the MMA
-            ok = wait0(bar_mi, ph_mi, pend_mi);
-            if (ok) issue_weight(g + 1);
+          issue_piece(tmem + 128 * (g & 1), sb + (ps.a == BUF_X ? kOffX : kOffH), sb + kOffW, idesc, !ps.first,
+                      ps.last ? su32(&bars.layer[g & 1]) : bar_part);
+          (ps.last ? pend_layer : pend_part) = true;
+          if (p == 0 && it > 0 && pq) {
+            stores_read();  // the last tile's Q
+            issue_h(tile_of(it));
+          }
+          if (ps.last) {
+            ok = mbar_wait(su32(&bars.layer[g & 1]), (g >> 1) & 1);
+            if (!ok) break;
+            pend_layer = false;
+            g++;
           } else {
-            pend_m = true;
+            ok = wait_on(bar_part, ph_part, pend_part);
+            if (!ok) break;
           }
+          issue_weight(it * NP + p + 1);
+          if (!pq && p == 4) issue_h(tile_of(it + 1));
+          if (!pq && p == 5) issue_x(tile_of(it + 1));
         }
-        if (!ok) fail_wait();
+        if (ok && pq) {
+          ok = wait_epilogues(g - 1);
+          if (!ok) break;
+          store(&a.tm_pq, kOffX, 0, row0);
+          stores_read();
+          issue_x(tile_of(it + 1));
+          ok = wait_epilogues(g);
+          if (!ok) break;
+          store(&a.tm_pq, kOffH, 128, row0);
+        }
       }
-      if (ps.epi == EPI_NONE) continue;
-      // the layer's bias to shared memory (the last epilogue is done)
-      const float *bias = a.piece[p].bias;
-      const int ncol = ps.epi == EPI_PQ ? 256 : ps.epi == EPI_OUT ? 16 : 128;
-      if (bias)
-        for (int c = tid; c < ncol; c += kThreads) s_bias[c] = bias[c];
-      __syncthreads();
-      if (s_abort) break;
-      bool ok = mbar_wait(bar_m, ph_m);
-      if (ok) {
-        ph_m ^= 1u;
-        if (tid == 0) pend_m = false;
-      } else {
-        fail_wait();
-      }
-      // Each thread polls on its own clock, so a wait can give up in some
-      // threads only.  The warp-wide TMEM loads below need the whole warp;
-      // s_abort, read after the next block barrier, stops every warp.
-      ok = __all_sync(0xffffffffu, ok);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (ok) {
-        // the MMA has read its operands: refill what it freed
-        if (tid == 0) {
-          if (ps.epi != EPI_PQ) issue_weight(g + 1);  // after a [P | Q] layer the slot stages Q first
-          if (next && a.mode == CHAIN_LAST) {
-            if (p == 4) issue_h(tile_of(it + 1));
-            if (p == 5) issue_x(tile_of(it + 1));
-          }
-        }
-        if (ps.epi == EPI_RESIDUAL) {
-          if (!mbar_wait(bar_h, ph_h_all)) fail_wait();
-          ph_h_all ^= 1u;
-        }
-        const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-        if (ps.epi == EPI_OUT) {
-          float v[16];
-          tmem_ld16(taddr, v);
-          const int grow = row0 + r;
+      // normal end or a failed wait: let every copy, store or MMA in flight
+      // land (bounded again).  An MMA that still has not completed may write
+      // the accumulator: its TMEM is then left allocated rather than freed
+      // under it.
+      bool mma_done = true;
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+      if (pend_x) mbar_wait(bar_x, ph_x);
+      if (pend_h) mbar_wait(bar_h, ph_h);
+      if (pend_w) mbar_wait(bar_w, ph_w);
+      if (pend_part && !mbar_wait(bar_part, ph_part)) mma_done = false;
+      if (pend_layer && !mbar_wait(su32(&bars.layer[g & 1]), (g >> 1) & 1)) mma_done = false;
+      if (!ok || !mma_done) atomicOr(a.err, ERR_TIMEOUT);
+      if (!mma_done) s_mma_pending = 1;
+    }
+    __syncwarp();
+  } else {
+    const int r = (warp & 3) * 32 + lane;  // tile row = TMEM lane of this thread
+    const int half = warp >> 2;            // columns [64 half, 64 half + 64): one atom
+    bool ok = true;
+    int g = 0;
+    for (int it = 0; ok && tile_of(it) < a.ntiles; it++) {
+      const int row0 = tile_of(it) * 128;
+      for (int l = 0; l < NL; l++, g++) {
+        const LayerSpec ls = layer_of(a.mode, l);
+        ok = mbar_wait(su32(&bars.layer[g & 1]), (g >> 1) & 1);
+        // h was written by TMA: its readers wait for its barrier themselves
+        if (ok && ls.epi == EPI_RESIDUAL) ok = mbar_wait(su32(&bars.h), it & 1);
+        // Each thread polls on its own clock, so a wait can give up in some
+        // threads only; the warp-wide TMEM loads below need the whole warp.
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t taddr = tmem + 128 * (g & 1) + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        const bool biased = bias_of(a, l) != nullptr;
+        if (ls.epi == EPI_OUT) {
+          if (half == 0) {
+            float v[16];
+            tmem_ld16(taddr, v);
+            const int grow = row0 + r;
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[j] += s_bias[j];
-          if (grow < a.n) {
-            float4 *dst = reinterpret_cast<float4 *>(a.out + (size_t)grow * 128);
+            for (int j = 0; j < 16; j++) v[j] += s_bias[l][j];
+            if (grow < a.n) {
+              float4 *dst = reinterpret_cast<float4 *>(a.out + (size_t)grow * 128);
 #pragma unroll
-            for (int j = 0; j < 4; j++) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          }
-        } else {
-          for (int c64 = 0; c64 < ncol; c64 += 64) {
-            float v[64];
-            tmem_ld64(taddr + c64, v);
-            if (bias)
-#pragma unroll
-              for (int j = 0; j < 64; j++) v[j] += s_bias[c64 + j];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-              float *w = v + 16 * q;
-              const int c0 = c64 + 16 * q;
-              if (ps.epi == EPI_RESIDUAL) {
-                float h[16];
-                smem_get16(sm + kOffH, r, c0, h);
-#pragma unroll
-                for (int j = 0; j < 16; j++) w[j] += h[j];
-                smem_put16(sm + kOffH, r, c0, w);
-              } else if (ps.epi == EPI_PQ) {
-                if (c0 < 128)
-                  smem_put16(sm + kOffX, r, c0, w);
-                else
-                  smem_put16(sm + kOffW, r, c0 - 128, w);
-              } else {
-                if (ps.relu)
-#pragma unroll
-                  for (int j = 0; j < 16; j++) w[j] = fmaxf(w[j], 0.0f);
-                smem_put16(sm + (ps.epi == EPI_H ? kOffH : kOffX), r, c0, w);
-              }
+              for (int j = 0; j < 4; j++) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
             }
           }
-        }
-      }
-      // shared-memory results -> visible to the next MMA and the TMA stores
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncthreads();
-      if (s_abort) {
-        stop = true;
-        continue;
-      }
-      const bool h_done = (ps.epi == EPI_RESIDUAL || ps.epi == EPI_H) && a.store_h;
-      if (tid == 0 && (h_done || ps.epi == EPI_PQ)) {
-        if (h_done) {
-          tma_store_box(&a.tm_hout, sb + kOffH, 0, row0);
-          tma_store_box(&a.tm_hout, sb + kOffH + kAtom, 64, row0);
-        }
-        if (ps.epi == EPI_PQ) {
-          tma_store_box(&a.tm_pq, sb + kOffX, 0, row0);
-          tma_store_box(&a.tm_pq, sb + kOffX + kAtom, 64, row0);
-          tma_store_box(&a.tm_pq, sb + kOffW, 128, row0);
-          tma_store_box(&a.tm_pq, sb + kOffW + kAtom, 192, row0);
-        }
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        if (ps.epi == EPI_PQ) {
-          // the stores have read X, h and the slot: refill them
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          issue_weight(g + 1);
-          if (next) {
-            issue_x(tile_of(it + 1));
-            if (has_h) issue_h(tile_of(it + 1));
+        } else {
+          float v[64];
+          tmem_ld64(taddr + 64 * half, v);
+          if (biased)
+#pragma unroll
+            for (int j = 0; j < 64; j++) v[j] += s_bias[l][64 * half + j];
+          uint8_t *buf = sm + (ls.epi == EPI_X ? kOffX : kOffH);
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            float *w = v + 16 * q;
+            const int c0 = 64 * half + 16 * q;
+            if (ls.epi == EPI_RESIDUAL) {
+              float h[16];
+              smem_get16(buf, r, c0, h);
+#pragma unroll
+              for (int j = 0; j < 16; j++) w[j] += h[j];
+            }
+            if (ls.relu)
+#pragma unroll
+              for (int j = 0; j < 16; j++) w[j] = fmaxf(w[j], 0.0f);
+            smem_put16(buf, r, c0, w);
           }
         }
+        // results -> visible to the next MMA and the TMA stores
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(su32(&bars.epi[g & 1]));
       }
-      if (ps.epi == EPI_PQ) __syncthreads();
     }
-  }
-  // normal end or a failed wait: let every copy, store or MMA in flight land
-  // (bounded again).  An MMA that still has not completed may write the
-  // accumulator: its TMEM is then left allocated rather than freed under it.
-  if (tid == 0) {
-    bool mma_done = true;
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-    if (pend_x) mbar_wait(bar_x, ph_x);
-    if (pend_h) mbar_wait(bar_h, ph_h);
-    if (pend_w) mbar_wait(bar_w, ph_w);
-    if (pend_mi && !mbar_wait(bar_mi, ph_mi)) mma_done = false;
-    if (pend_m && !mbar_wait(bar_m, ph_m)) mma_done = false;
-    if (!mma_done) {
-      fail_wait();
-      s_mma_pending = 1;
-    }
+    if (!ok) atomicOr(a.err, ERR_TIMEOUT);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0 && !s_mma_pending)
+  if (warp == kEpiWarps && !s_mma_pending)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256));
 }
 

@@ -45,9 +45,9 @@ constexpr int kMaxDeg = UPH_SUR_MAX_DEGREE;
 constexpr int kMaxRounds = UPH_SUR_MAX_ROUNDS;
 constexpr int kEdgeThreads = 256;           // 8 warps
 // fixed grid (per-warp partials in a fixed order) of one wave: the edge
-// kernels take 80 registers x 256 threads, so three blocks fit an SM's 64K
-// registers; a fourth block per SM would run as a second, mostly empty wave
-constexpr int kEdgeBlocks = 148 * 3, kEdgeBwdBlocks = 148 * 2;
+// kernels take up to 128 registers x 256 threads, so two blocks fill an SM's
+// 64K registers; a third block per SM would run as a second, mostly empty wave
+constexpr int kEdgeBlocks = 148 * 2;
 constexpr int kSplitMax = 148;              // split-K CTAs of one weight-gradient GEMM tile
 constexpr int kLossBlocks = 148;
 constexpr int kMaxBins = 4096;
@@ -97,18 +97,6 @@ ParamOff param_layout(int rounds)
 }
 
 // ---- small device helpers ------------------------------------------------------
-__device__ __forceinline__ void load_bf16x4(const bf16 *p, float out[4])
-{
-  const uint2 raw = *reinterpret_cast<const uint2 *>(p);
-  const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162 *>(&raw.x);
-  const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162 *>(&raw.y);
-  const float2 fa = __bfloat1622float2(a), fb = __bfloat1622float2(b);
-  out[0] = fa.x;
-  out[1] = fa.y;
-  out[2] = fb.x;
-  out[3] = fb.y;
-}
-
 __device__ __forceinline__ void store_bf16x4(bf16 *p, const float v[4])
 {
   __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]);
@@ -169,13 +157,22 @@ __device__ __forceinline__ f32x2 relu2(f32x2 v)
 // order (cells row by row, ids ascending inside a cell: deterministic), and
 // their edge features in FP32: (dx, dy, r) / R and the density difference
 // (rho_j - rho_i) / rho_unit
-__global__ void k_sur_graph(DevParams G, const double *__restrict__ x, const double *__restrict__ y,
-                            const double *__restrict__ rho, double rho_unit, int n, const int *__restrict__ cell_of,
-                            const int *__restrict__ start, const int *__restrict__ list, double R,
-                            int *__restrict__ nbr, float4 *__restrict__ ef, int *__restrict__ deg, unsigned *err)
+//
+// Eight lanes per node test eight candidates at a time and place the hits by
+// a ballot: 59 us at 207,000 nodes of some 60 candidates (109 with a thread per
+// node, which waits for one chain of loads per four candidates and stores its
+// hits 16 bytes at a time), bound by the latency of those loads.
+constexpr int kGraphThreads = 128, kGraphLanes = 8;
+__global__ void __launch_bounds__(kGraphThreads) k_sur_graph(
+    DevParams G, const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ rho,
+    double rho_unit, int n, const int *__restrict__ cell_of, const int *__restrict__ start,
+    const int *__restrict__ list, double R, int *__restrict__ nbr, float4 *__restrict__ ef, int *__restrict__ deg,
+    unsigned *err)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const int node = (blockIdx.x * kGraphThreads + threadIdx.x) / kGraphLanes;
+  const int lane = threadIdx.x & 31, sub = lane & (kGraphLanes - 1), shift = lane & ~(kGraphLanes - 1);
+  const bool live = node < n;  // a group without a node keeps its warp's loops uniform
+  const int i = live ? node : n - 1;
   const double xi = x[i], yi = y[i], ri = rho[i];
   const double r2cut = R * R;
   // features by multiplication with reciprocals (no FP64 division or square
@@ -183,41 +180,55 @@ __global__ void k_sur_graph(DevParams G, const double *__restrict__ x, const dou
   const double inv_R = 1.0 / R, inv_R2 = 1.0 / r2cut, inv_rho_unit = 1.0 / rho_unit;
   const int c = cell_of[i];
   const int cx = c % G.ncx, cy = c / G.ncx;
+  const int x0 = max(cx - 1, 0), x1 = min(cx + 1, G.ncx - 1);
+  // the three rows' candidates as one range of [0, end[2])
+  int first[3], end[3], total = 0;
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const int yy = cy + r - 1;
+    int a = 0, b = 0;
+    if (live && yy >= 0 && yy < G.ncy) {
+      a = start[yy * G.ncx + x0];
+      b = start[yy * G.ncx + x1 + 1];
+    }
+    first[r] = a - total;
+    total += b - a;
+    end[r] = total;
+  }
+  const int steps = __reduce_max_sync(0xffffffffu, total);
   int cnt = 0;
-  for (int oy = -1; oy <= 1; oy++) {
-    const int yy = cy + oy;
-    if (yy < 0 || yy >= G.ncy) continue;
-    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, G.ncx - 1);
-    const int a = start[yy * G.ncx + x0], b = start[yy * G.ncx + x1 + 1];
-    // four candidates per pass: their position loads are independent
-    for (int k0 = a; k0 < b; k0 += 4) {
-      int jj[4];
-      double cx4[4], cy4[4];
+  constexpr int kU = 2;  // candidates of a lane in flight
+  for (int k0 = 0; k0 < steps; k0 += kU * kGraphLanes) {
+    int jj[kU];
+    double xj[kU], yj[kU], rj[kU];
 #pragma unroll
-      for (int u = 0; u < 4; u++) jj[u] = k0 + u < b ? list[k0 + u] : -1;
+    for (int u = 0; u < kU; u++) {
+      const int k = k0 + u * kGraphLanes + sub;
+      jj[u] = k < total ? list[k + (k < end[0] ? first[0] : k < end[1] ? first[1] : first[2])] : -1;
+    }
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        cx4[u] = jj[u] >= 0 ? x[jj[u]] : 0.0;
-        cy4[u] = jj[u] >= 0 ? y[jj[u]] : 0.0;
+    for (int u = 0; u < kU; u++) {
+      const int j = max(jj[u], 0);
+      xj[u] = x[j];
+      yj[u] = y[j];
+      rj[u] = rho[j];
+    }
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+      const double dx = xj[u] - xi, dy = yj[u] - yi;
+      const double r2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+      const bool hit = jj[u] >= 0 && r2 > DBL_EPSILON && r2 < r2cut;
+      const unsigned hits = (__ballot_sync(0xffffffffu, hit) >> shift) & ((1u << kGraphLanes) - 1);
+      const int at = cnt + __popc(hits & ((1u << sub) - 1));
+      if (hit && at < kMaxDeg) {
+        nbr[(size_t)i * kMaxDeg + at] = jj[u];
+        ef[(size_t)i * kMaxDeg + at] = make_float4((float)(dx * inv_R), (float)(dy * inv_R),
+                                                   sqrtf((float)(r2 * inv_R2)), (float)((rj[u] - ri) * inv_rho_unit));
       }
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int j = jj[u];
-        if (j < 0) continue;
-        const double dx = cx4[u] - xi, dy = cy4[u] - yi;
-        const double r2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-        if (r2 > DBL_EPSILON && r2 < r2cut) {
-          if (cnt < kMaxDeg) {
-            nbr[(size_t)i * kMaxDeg + cnt] = j;
-            ef[(size_t)i * kMaxDeg + cnt] = make_float4((float)(dx * inv_R), (float)(dy * inv_R),
-                                                        sqrtf((float)(r2 * inv_R2)),
-                                                        (float)((rho[j] - ri) * inv_rho_unit));
-          }
-          cnt++;
-        }
-      }
+      cnt += __popc(hits);
     }
   }
+  if (!live || sub != 0) return;
   if (cnt > kMaxDeg) {
     atomicOr(err, ERR_NEIGHBOR_OVERFLOW);
     cnt = kMaxDeg;
@@ -245,9 +256,8 @@ __global__ void k_sur_features(int n, const double *__restrict__ u, const double
   if (!isfinite(f[0]) || !isfinite(f[1]) || !isfinite(f[2])) atomicOr(err, ERR_NAN);
   __align__(16) __nv_bfloat162 h[4];
   for (int k = 0; k < 4; k++) h[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
-  uint4 *row = reinterpret_cast<uint4 *>(F + (size_t)i * kFeat);
-  row[0] = *reinterpret_cast<uint4 *>(&h[0]);
-  for (int k = 1; k < kFeat / 8; k++) row[k] = make_uint4(0u, 0u, 0u, 0u);
+  // the row's other columns are zero from its allocation on
+  *reinterpret_cast<uint4 *>(F + (size_t)i * kFeat) = *reinterpret_cast<uint4 *>(&h[0]);
 }
 
 // ---- edge layer -----------------------------------------------------------------
@@ -278,10 +288,12 @@ __device__ __forceinline__ void cp_wait()
 // per node, lane l of the half owning channels [8l, 8l + 8) as four packed
 // FP32 pairs.  A partner costs one shared broadcast read of its record and one
 // 16-byte gather of its Q row; partners are summed in graph order.  Bound by
-// issue and by the gathers' latency at 24 warps per SM: 82 us at 83,000 nodes
-// and 187 at 207,000 (83 and 190 with a node's records fetched when its turn
-// comes; 86 and 203 with the nodes in cell order, which hits L1 no more often).
-__global__ void __launch_bounds__(kEdgeThreads, 3) k_sur_edge_fwd(int n, const bf16 *__restrict__ PQ,
+// the FP32 pipe (56 % active; 105 us of its cycles at 207,000 nodes of 20
+// partners) and by what it waits for: 175 us there with eight rows in flight
+// at 16 warps per SM, 187 with four rows at 24 warps, 228 to 250 with a warp
+// per node (twice the broadcasts and moves per channel), 175 to 205 with eight
+// lanes per node, 203 with the nodes in cell order.
+__global__ void __launch_bounds__(kEdgeThreads, 2) k_sur_edge_fwd(int n, const bf16 *__restrict__ PQ,
                                                                  const float *__restrict__ we,
                                                                  const int *__restrict__ nbr,
                                                                  const float4 *__restrict__ ef,
@@ -350,6 +362,13 @@ __global__ void __launch_bounds__(kEdgeThreads, 3) k_sur_edge_fwd(int n, const b
     };
     auto q_row = [&](int k) { return *reinterpret_cast<const uint4 *>(PQ + (size_t)N.j[k] * 2 * kLat + kLat + c0); };
     int k = 0;
+    for (; k + 8 <= d; k += 8) {
+      uint4 qv[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) qv[u] = q_row(k + u);
+#pragma unroll
+      for (int u = 0; u < 8; u++) edge(N.rec[k + u], qv[u]);
+    }
     for (; k + 4 <= d; k += 4) {
       uint4 qv[4];
 #pragma unroll
@@ -912,8 +931,10 @@ uph_status prepare(uph_surrogate *s, const NodesView &nv)
   launch_exclusive_scan(g.count, g.start, (int)ncell, g.block_sums, q);
   launch_cell_scatter(g, 0, nv.n, q);
   launch_cell_sort_segments(g, s->d_err, q);
-  k_sur_graph<<<(nv.n + 127) / 128, 128, 0, q>>>(G, nv.x, nv.y, nv.rho, s->cfg.rho0 * s->cfg.edge_rho_scale, nv.n,
-                                                 g.cell_of, g.start, g.list, R, s->nbr, s->ef, s->deg, s->d_err);
+  constexpr int kNodes = kGraphThreads / kGraphLanes;
+  k_sur_graph<<<(nv.n + kNodes - 1) / kNodes, kGraphThreads, 0, q>>>(
+      G, nv.x, nv.y, nv.rho, s->cfg.rho0 * s->cfg.edge_rho_scale, nv.n, g.cell_of, g.start, g.list, R, s->nbr, s->ef,
+      s->deg, s->d_err);
   k_sur_features<<<(nv.n + 255) / 256, 256, 0, q>>>(nv.n, nv.u, nv.v, nv.rho, nv.itype, s->cfg.vel_scale,
                                                      s->cfg.rho0, s->cfg.rho_scale, s->F, s->d_err);
   UPH_CUDA(cudaGetLastError());
@@ -1191,9 +1212,9 @@ uph_status backward_net(uph_surrogate *s, int n)
       c.c_f32 = s->dS; c.ldc = kLat;
       TRYS(run(s, c));
     }
-    k_sur_edge_bwd<<<kEdgeBwdBlocks, kEdgeThreads, 0, q>>>(n, s->PQ[r], s->w + ro.we, s->nbr, s->ef, s->deg, s->dS,
-                                                        s->dPQ, s->wepart);
-    sum_rows(s->wepart, kEdgeBwdBlocks, kLat * 4, G + ro.we, q);
+    k_sur_edge_bwd<<<kEdgeBlocks, kEdgeThreads, 0, q>>>(n, s->PQ[r], s->w + ro.we, s->nbr, s->ef, s->deg, s->dS,
+                                                         s->dPQ, s->wepart);
+    sum_rows(s->wepart, kEdgeBlocks, kLat * 4, G + ro.we, q);
     TRYS(wgrad(s, s->dPQ, 2 * kLat, 2 * kLat, s->cat[r], 2 * kLat, kLat, n, G + ro.pq_w, G + ro.pq_b));
     {
       GemmCall c;  // dh += dPQ . W_pq, and its BF16 copy for the next round down
@@ -1326,6 +1347,7 @@ extern "C" uph_status uph_sur_create(const uph_sur_config *cfg, int32_t node_cap
     return tr;
   }
   cudaMemset(s->d_err, 0, sizeof(unsigned));
+  cudaMemset(s->F, 0, sizeof(bf16) * c * kFeat);
   cudaMemset(s->w, 0, sizeof(float) * P);
   cudaMemset(s->wb, 0, sizeof(bf16) * P);
   cudaMemset(s->am, 0, sizeof(float) * P);
