@@ -356,12 +356,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_node_chain(const __grid_constan
         }
         return ok;
       };
-      // piece q % NP of iteration q / NP into the weight slot
-      auto issue_weight = [&](int q) {
-        if (tile_of(q / NP) >= a.ntiles) return;
+      // the weight piece into its slot: one contiguous image of two atoms
+      auto issue_weight = [&](int p) {
         mbar_expect(bar_w, kPieceBytes);
-        bulk_load(sb + kOffW, a.piece[q % NP].img, kAtom, bar_w);
-        bulk_load(sb + kOffW + kAtom, a.piece[q % NP].img + kAtom, kAtom, bar_w);
+        bulk_load(sb + kOffW, a.piece[p].img, kPieceBytes, bar_w);
         pend_w = true;
       };
       auto issue_x = [&](int tile) {
@@ -422,7 +420,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_node_chain(const __grid_constan
             ok = wait_on(bar_part, ph_part, pend_part);
             if (!ok) break;
           }
-          issue_weight(it * NP + p + 1);
+          if (p + 1 < NP)
+            issue_weight(p + 1);
+          else if (tile_of(it + 1) < a.ntiles)
+            issue_weight(0);
           if (!pq && p == 4) issue_h(tile_of(it + 1));
           if (!pq && p == 5) issue_x(tile_of(it + 1));
         }
