@@ -552,6 +552,10 @@ __device__ __forceinline__ void step_run(const CellBuildArgs &C, const SlotArray
 {
   const DevParams &P = C.P;
   const CellGrid &G = C.G;
+  // nothing of the launch before is read or overwritten above this line; the
+  // next launch's blocks may take the places that this one's blocks leave
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   StepMode mode = step_begin(C, A, smem);
   step_walls(P, F);
   if (mode == STEP_RECORD && !step_record<kBrute>(C, S, A, smem)) mode = STEP_FAILED;
@@ -592,7 +596,23 @@ uph_status launch_step(size_t smem, const DevParams &P, const SlotArrays &S, con
   CellBuildArgs C = cell_build_args(P, S.x, S.y, 0, P.n, G, err, false);
   C.rebuild = P.rebuild;
   C.P.rebuild = A.moved;
-  kStep<<<std::max(1, std::min(most, P.ntx * (P.ncy / P.tile))), kTileThreads, smem, s>>>(C, S, F, A);
+  // The next step's blocks are set up while this one's last blocks run
+  // (step_run waits for the launch before it): 22.3 against 23.1 us a step of 5,000
+  // particles, 45 against 47 of 61,000.  In a captured graph, whose nodes follow each other faster,
+  // plain edges are the better ones: 36.6 against 37.6 us a step.
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  UPH_CUDA(cudaStreamIsCapturing(s, &capturing));
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(std::max(1, std::min(most, P.ntx * (P.ncy / P.tile))));
+  cfg.blockDim = dim3(kTileThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = capturing == cudaStreamCaptureStatusNone ? 1 : 0;
+  UPH_CUDA(cudaLaunchKernelEx(&cfg, kStep, C, S, F, A));
   return UPH_OK;
 }
 
