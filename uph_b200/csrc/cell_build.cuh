@@ -250,50 +250,68 @@ __device__ __forceinline__ bool cell_build_phases(const CellBuildArgs &A, const 
       }))
     return false;
 
-  // 2. chunk scans
+  // 2. chunk scans.  Each warp takes a contiguous share of the chunk: it adds
+  // the share up, and scans it once the shares before it are known, so that a
+  // warp has kU words in flight and never waits for another inside its share.
+  // 9.7 million cells over 296 parts of 256 threads: 25 us; 137 with the whole
+  // block scanning 2,048 cells at a time.
   if (!ph.run(1, [&](int b) {
         const int c0 = min(b * chunk, ncell), c1 = min(c0 + chunk, ncell);
-        int carry = 0;
-        for (int base = c0; base < c1; base += nt * 8) {
-          const int c = base + t * 8;
-          int v[8], sum = 0;
-          if (c + 8 <= c1) {
-            *reinterpret_cast<int4 *>(v) = *reinterpret_cast<const int4 *>(cnt + c);
-            *reinterpret_cast<int4 *>(v + 4) = *reinterpret_cast<const int4 *>(cnt + c + 4);
-            const int4 z = make_int4(0, 0, 0, 0);
-            *reinterpret_cast<int4 *>(cnt + c) = z;
-            *reinterpret_cast<int4 *>(cnt + c + 4) = z;
-          } else {
+        const int lane = t & 31, wid = t >> 5, nw = nt >> 5;
+        const int share = ((chunk + nw - 1) / nw + 3) & ~3;
+        const int w0 = min(c0 + wid * share, c1), w1 = min(w0 + share, c1);
+        const int whole = w0 + ((w1 - w0) & ~3);  // the words; what is left is the grid's last cells
+        int sum = 0;
+        for (int c = w0 + 4 * lane; c < whole; c += 128 * 2 * kU) {
+          int4 v[2 * kU];
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-              v[j] = 0;
-              if (c + j < c1) {
-                v[j] = cnt[c + j];
-                cnt[c + j] = 0;
-              }
+          for (int u = 0; u < 2 * kU; u++)
+            v[u] = c + 128 * u < whole ? *reinterpret_cast<const int4 *>(cnt + c + 128 * u) : make_int4(0, 0, 0, 0);
+#pragma unroll
+          for (int u = 0; u < 2 * kU; u++) sum += v[u].x + v[u].y + v[u].z + v[u].w;
+        }
+        if (whole + lane < w1) sum += cnt[whole + lane];
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0) s_wt[wid] = sum;
+        __syncthreads();
+        int run = 0, total = 0;
+        for (int k = 0; k < nw; k++) {
+          const int v = s_wt[k];
+          if (k < wid) run += v;
+          total += v;
+        }
+        for (int base = w0; base < whole; base += 128 * kU) {
+          int4 v[kU];
+#pragma unroll
+          for (int u = 0; u < kU; u++) {
+            const int c = base + 128 * u + 4 * lane;
+            v[u] = c < whole ? *reinterpret_cast<const int4 *>(cnt + c) : make_int4(0, 0, 0, 0);
+          }
+#pragma unroll
+          for (int u = 0; u < kU; u++) {
+            const int c = base + 128 * u + 4 * lane;
+            const int mine = v[u].x + v[u].y + v[u].z + v[u].w;
+            int incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const int up = __shfl_up_sync(0xffffffffu, incl, o);
+              if (lane >= o) incl += up;
+            }
+            const int e0 = run + incl - mine, e1 = e0 + v[u].x, e2 = e1 + v[u].y;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+            if (c < whole) {
+              *reinterpret_cast<int4 *>(fill + c) = make_int4(e0, e1, e2, e2 + v[u].z);
+              *reinterpret_cast<int4 *>(cnt + c) = make_int4(0, 0, 0, 0);
             }
           }
-#pragma unroll
-          for (int j = 0; j < 8; j++) sum += v[j];
-          int total;
-          int run = block_exclusive_scan<int>(sum, s_wt, total) + carry;
-#pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const int n = v[j];
-            v[j] = run;
-            run += n;
-          }
-          if (c + 8 <= c1) {
-            *reinterpret_cast<int4 *>(fill + c) = *reinterpret_cast<const int4 *>(v);
-            *reinterpret_cast<int4 *>(fill + c + 4) = *reinterpret_cast<const int4 *>(v + 4);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-              if (c + j < c1) fill[c + j] = v[j];
-          }
-          carry += total;
         }
-        if (t == 0) A.G.totals[b] = carry;
+        if (lane == 0)
+          for (int c = whole; c < w1; c++) {
+            fill[c] = run;
+            run += cnt[c];
+            cnt[c] = 0;
+          }
+        if (t == 0) A.G.totals[b] = total;
       }))
     return false;
 
