@@ -516,12 +516,13 @@ __device__ __forceinline__ void stream_record(const DevParams &P, const SlotArra
   }
 }
 
-// The recording of every tile that holds a particle: a CTA per tile where
-// that is few rounds of the grid, for the shorter chain, else a warp per
-// tile, for the more tiles in flight.  us on a stirred dam break: 61,000
-// particles (390 tiles, 296 CTAs) 27 against 84, 300,000 (1,600 tiles) 100
-// against 86, 2,000,000 (9,600 tiles) 630 against 404 (before the lists went
-// through the ring).
+// The recording of every tile that holds a particle: a warp per tile, for the
+// more tiles in flight, in whole rounds of the grid's warps, and a CTA per
+// tile, for the shorter chain, where what is left is few rounds of the grid.
+// us on a stirred dam break: 61,000 particles (390 tiles, 296 CTAs) 25 by
+// CTAs, 84 by warps; 300,000 (1,600 tiles) 100 against 72; 2,000,000 (9,600
+// tiles, four rounds of warps and 130 tiles) 285 with the last ones by CTAs,
+// 327 without.
 template <bool kBrute>
 __device__ __forceinline__ bool step_record(const CellBuildArgs &C, const SlotArrays &S, const StepArgs &A,
                                             unsigned char *smem)
@@ -532,15 +533,16 @@ __device__ __forceinline__ bool step_record(const CellBuildArgs &C, const SlotAr
   const int nlive = *(volatile int *)G.st.nlive;
   const volatile int *live = G.st.live;
   const TicketPhases ph{A.phases, C.err};
+  constexpr int kWarps = kTileThreads / 32;
+  const int round = (int)gridDim.x * kWarps, rest = nlive % round;
+  const int by_warps = rest <= 4 * (int)gridDim.x ? nlive - rest : nlive;
   return ph.run(4, [&](int b) {
-    if (nlive <= 4 * (int)gridDim.x) {
-      for (int t = b; t < nlive; t += gridDim.x) stream_record<kBrute, kTileThreads>(C.P, S, G, live[t], R[0], ring);
-    } else {
-      constexpr int kWarps = kTileThreads / 32;
-      const int w = threadIdx.x >> 5;
-      for (int t = b * kWarps + w; t < nlive; t += gridDim.x * kWarps)
-        stream_record<kBrute, 32>(C.P, S, G, live[t], R[w], ring);
-    }
+    const int w = threadIdx.x >> 5;
+    for (int t = b * kWarps + w; t < by_warps; t += round)
+      stream_record<kBrute, 32>(C.P, S, G, live[t], R[w], ring);
+    if (by_warps < nlive) __syncthreads();
+    for (int t = by_warps + b; t < nlive; t += gridDim.x)
+      stream_record<kBrute, kTileThreads>(C.P, S, G, live[t], R[0], ring);
   });
 }
 
@@ -597,9 +599,10 @@ uph_status launch_step(size_t smem, const DevParams &P, const SlotArrays &S, con
   C.rebuild = P.rebuild;
   C.P.rebuild = A.moved;
   // The next step's blocks are set up while this one's last blocks run
-  // (step_run waits for the launch before it): 22.3 against 23.1 us a step of 5,000
-  // particles, 45 against 47 of 61,000.  In a captured graph, whose nodes follow each other faster,
-  // plain edges are the better ones: 36.6 against 37.6 us a step.
+  // (step_run waits for the launch before it): 22.3 against 23.1 us a
+  // step of 5,000 particles, 45 against 47 of 61,000.  In a captured graph,
+  // whose nodes follow each other faster, plain edges are the better ones:
+  // 18.3 against 18.8 us a step of 5,000.
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   UPH_CUDA(cudaStreamIsCapturing(s, &capturing));
   cudaLaunchAttribute early{};
