@@ -28,11 +28,13 @@
 // the running epilogue (N1's h half, W_Q, the next tile's first) is multiplied
 // beside it.
 //
-// Bound by the chain of a tile (MMA, epilogue, next MMA), which the SM's two
-// CTAs overlap, and by one weight piece's way from L2 per MMA; the tensor pipe
-// is busy for some 20 us of a round at 207,000 nodes.  A round there: NEWR us
-// (encoder NEWE, last round NEWL), against 114 (90, 91) with four warps that
-// waited for every load, MMA and store in turn.
+// Bound by the chain of a tile (a layer's MMA some 1,200 cycles, its epilogue
+// 3,000, then [P | Q] out and the next operand in, 4,000), which the SM's two
+// CTAs overlap; the tensor pipe is busy for some 20 us of a round at 207,000
+// nodes.  A round there: 88 us (encoder 69, last round 76), against 114 (90,
+// 91) with four warps that waited for every load, MMA and store in turn, and
+// 89 (66, 86) with one CTA per SM whose two tiles share a ring of three weight
+// pieces: both tiles then end together.
 //
 // The arithmetic is that of the unfused path (tc_gemm.cu) step for step --
 // the same K order of MMAs, FP32 bias then residual, the same BF16 rounding
