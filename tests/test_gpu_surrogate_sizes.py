@@ -62,11 +62,13 @@ def test_gradients_at_tile_edges(n):
         assert e <= 5e-2, (name, e)
 
 
-@pytest.mark.parametrize("M,splits,accumulate", [(200, 5, 0), (200, 5, 1), (256, 3, 1), (77, 1, 1)])
-def test_split_products_of_partial_tiles(M, splits, accumulate):
+@pytest.mark.parametrize("M,splits,accumulate,skew", [(200, 5, 0, 0), (200, 5, 1, 0), (256, 3, 1, 0), (77, 1, 1, 0),
+                                                      (200, 5, 1, 1)])
+def test_split_products_of_partial_tiles(M, splits, accumulate, skew):
     """M off the 128-row tile (partials are not whole boxes), 11 slices of K
-    over splits that do not divide them, a sum added to what is there; the
-    bound is the summation order's, 1e-3 of the largest value."""
+    over splits that do not divide them, a sum added to what is there, a
+    result off the 16-byte boundary; the bound is the summation order's, 1e-3
+    of the largest value."""
     import ctypes as C
 
     from test_gpu_tc_gemm import _lib
@@ -75,7 +77,7 @@ def test_split_products_of_partial_tiles(M, splits, accumulate):
     gen = torch.Generator(device="cuda").manual_seed(M)
     A = torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
     B = torch.randn(N, K, device="cuda", generator=gen).to(torch.bfloat16)
-    c = torch.randn(M + 8, N, device="cuda", generator=gen)
+    c = torch.randn((M + 8) * N + 4, device="cuda", generator=gen)[skew:skew + (M + 8) * N].view(M + 8, N)
     before = c.clone()
     part = torch.empty(splits * M * N, device="cuda")
     err = torch.zeros(1, dtype=torch.int32, device="cuda")

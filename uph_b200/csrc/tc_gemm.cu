@@ -480,7 +480,10 @@ __global__ void __launch_bounds__(256) k_splitk_reduce(const float *__restrict__
   __syncthreads();
   if (grp != 0 || i >= n) return;
   float *dst = (is_col ? col_out : out) + i;
-  float4 t = !is_col && accumulate ? *reinterpret_cast<const float4 *>(dst) : make_float4(0.f, 0.f, 0.f, 0.f);
+  // the caller's result need not lie on a 16-byte boundary
+  const bool words = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+  float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (!is_col && accumulate) t = words ? *reinterpret_cast<const float4 *>(dst) : make_float4(dst[0], dst[1], dst[2], dst[3]);
 #pragma unroll
   for (int k = 0; k < kReduceGroups; k++) {
     t.x += red[k][l].x;
@@ -488,7 +491,14 @@ __global__ void __launch_bounds__(256) k_splitk_reduce(const float *__restrict__
     t.z += red[k][l].z;
     t.w += red[k][l].w;
   }
-  *reinterpret_cast<float4 *>(dst) = t;
+  if (words) {
+    *reinterpret_cast<float4 *>(dst) = t;
+  } else {
+    dst[0] = t.x;
+    dst[1] = t.y;
+    dst[2] = t.z;
+    dst[3] = t.w;
+  }
 }
 
 uph_status launch_tc_gemm(const GemmCall &c, cudaStream_t s)
