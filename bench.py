@@ -250,7 +250,7 @@ def gpu_arm(args, rank, world, local_rank):
     peak, peak_kind = load_peaks()
     achieved = pass_bytes / pass_avg_s / 1e9 if pass_avg_s > 0 else 0.0
     # DRAM read + write bytes of one launch from the committed ncu capture
-    # (profiles/rate_pass_ref_fp64_hydrostatic500k.md)
+    # (profiles/step_streaming_tank500k.md)
     # and its FP64-pipe activity, the compute roof this kernel is held by
     traffic = None
     fp64_active = None
@@ -696,7 +696,7 @@ def main():
                    "parallelism": "replicas" if world > 1 else "single GPU"},
         "roofline": {"bound": "hbm", "achieved": r["achieved"], "peak": r["peak"], "unit": "GB/s",
                      "frac": r["achieved"] / r["peak"], "traffic": r["traffic"],
-                     "kernel": "rate pass (k_ref_pass)", "bytes_per_launch": r["pass_bytes"],
+                     "kernel": "step (k_ref_step: list build where due, rate pass, leapfrog)", "bytes_per_launch": r["pass_bytes"],
                      "avg_launch_ms": r["pass_avg_s"] * 1e3, "peak_source": r["peak_kind"],
                      "fp64_pipe_active_ncu": r["fp64_active"]},
         "cpu_baseline": cpu,
