@@ -406,9 +406,9 @@ __device__ __forceinline__ f32x2 where_positive(f32x2 z, f32x2 v)
 // symmetric and e_ba = (-e_ab.x, -e_ab.y, e_ab.z)).  A warp per node, lane l
 // owning channels [4l, 4l + 4) as two packed FP32 pairs; the rows of four
 // partners (1 KB each: P, Q, dS) are in flight at a time.  Bound by issue and
-// the gathers' latency: 207 us at 83,000 nodes, against 271 with scalar
-// arithmetic under branches and one partner's rows at a time (246 with that and
-// the nodes in cell order).
+// the gathers' latency: 194 us at 83,000 nodes, against 271 with scalar
+// arithmetic under branches and one partner's rows at a time; 207 with a
+// guarded last group of partners instead of shorter groups.
 __global__ void __launch_bounds__(kEdgeThreads, 2) k_sur_edge_bwd(int n, const bf16 *__restrict__ PQ,
                                                                    const float *__restrict__ we,
                                                                    const int *__restrict__ nbr,
@@ -489,21 +489,37 @@ __global__ void __launch_bounds__(kEdgeThreads, 2) k_sur_edge_bwd(int n, const b
         dq[q] = add2(dq[q], where_positive(y, sb[q]));
       }
     };
-    constexpr int kU = 4;
-    for (int k = 0; k < d; k += kU) {
-      uint2 pr[kU], qr[kU];
-      float4 ds[kU];
+    struct Rows {
+      uint2 p, q;
+      float4 ds;
+    };
+    auto rows = [&](int k) {
+      const int b = N.j[k];
+      const bf16 *row = PQ + (size_t)b * 2 * kLat + c0;
+      Rows r;
+      r.p = *reinterpret_cast<const uint2 *>(row);
+      r.q = *reinterpret_cast<const uint2 *>(row + kLat);
+      r.ds = *reinterpret_cast<const float4 *>(dS + (size_t)b * kLat + c0);
+      return r;
+    };
+    int k = 0;
+    for (; k + 4 <= d; k += 4) {
+      Rows r[4];
 #pragma unroll
-      for (int u = 0; u < kU; u++) {
-        const int b = N.j[min(k + u, d - 1)];
-        const bf16 *row = PQ + (size_t)b * 2 * kLat + c0;
-        pr[u] = *reinterpret_cast<const uint2 *>(row);
-        qr[u] = *reinterpret_cast<const uint2 *>(row + kLat);
-        ds[u] = *reinterpret_cast<const float4 *>(dS + (size_t)b * kLat + c0);
-      }
+      for (int u = 0; u < 4; u++) r[u] = rows(k + u);
 #pragma unroll
-      for (int u = 0; u < kU; u++)
-        if (k + u < d) edge(N.rec[k + u], pr[u], qr[u], ds[u]);
+      for (int u = 0; u < 4; u++) edge(N.rec[k + u], r[u].p, r[u].q, r[u].ds);
+    }
+    for (; k + 2 <= d; k += 2) {
+      Rows r[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) r[u] = rows(k + u);
+#pragma unroll
+      for (int u = 0; u < 2; u++) edge(N.rec[k + u], r[u].p, r[u].q, r[u].ds);
+    }
+    for (; k < d; k++) {
+      const Rows r = rows(k);
+      edge(N.rec[k], r.p, r.q, r.ds);
     }
     float v[4];
     unpack2(dp[0], v[0], v[1]);
