@@ -54,6 +54,16 @@ uph_status uph_tc_gemm_bf16(const void *A, int32_t lda, const void *B, int32_t l
                             int32_t K, const float *bias, int32_t relu, float *c_f32, void *c_bf16, int32_t ldc,
                             int32_t splits, float *partials, int32_t accumulate, unsigned *err, void *stream);
 
+/* The row product (splits == 1) with the whole epilogue the training products
+ * use, in order: + bias[N], + a BF16 residual, + the old c_f32 (accumulate),
+ * ReLU, zero where a BF16 mask is not positive; then FP32 and/or BF16 output.
+ * residual and mask ([M x ldc], 16-byte aligned) may be NULL, and may be given
+ * together and with accumulate. */
+uph_status uph_tc_gemm_bf16_epilogue(const void *A, int32_t lda, const void *B, int32_t ldb, int32_t M, int32_t N,
+                                     int32_t K, const float *bias, const void *residual, int32_t accumulate,
+                                     int32_t relu, const void *mask, float *c_f32, void *c_bf16, int32_t ldc,
+                                     unsigned *err, void *stream);
+
 /* Failure-detection self test of the tensor-core kernels' bounded waits: one
  * 128 x 128 x 64 tile (A, B device BF16 [128 x 64], c_f32 device [128 x 128])
  * whose CTA first waits on an mbarrier that nothing arrives at.  The wait

@@ -60,7 +60,7 @@ constexpr long long kWaitLimit = 1LL << 26;     // poll cap; the time bound is k
 struct TcGemmArgs {
   CUtensorMap tm_a, tm_b;
   // the FP32 result (or its partials), the BF16 result and the BF16 matrix
-  // the epilogue reads (residual or mask)
+  // the epilogue reads (the residual, else the mask)
   CUtensorMap tm_c32, tm_c16, tm_e16;
   int a_trans, b_trans;      // operand stored as [K x rows] (rows contiguous) instead of [rows x K]
   int M, N, K;               // K multiple of 64, N multiple of 128
@@ -69,6 +69,8 @@ struct TcGemmArgs {
   int relu;
   int masked;                // zero the result where tm_e16 <= 0
   int residual;              // add tm_e16 after the bias
+  const __nv_bfloat16 *mask;  // the mask beside a residual, read by the threads, or null
+  int ldm;
   int accumulate;            // add the result to tm_c32's contents
   int c32, c16;              // write tm_c32 / tm_c16
   float *partials;           // split-K whose tiles are not whole boxes: [splits][M][N] FP32 stored by the threads
@@ -207,7 +209,10 @@ __device__ __forceinline__ uint32_t tc_idesc()
       cute::UMMA::make_instr_desc<cute::bfloat16_t, cute::bfloat16_t, float, kTcM, kTcN, A, B>());
 }
 
-template <int kStages>
+// kBoth: the old result and a BF16 matrix are read, or a residual and a mask
+// (forms that no layer of the network needs: in the layers' own kernel their
+// checks and addresses would cost 0.6 us a product)
+template <int kStages, bool kBoth>
 __global__ void __launch_bounds__(128) k_tc_gemm(const __grid_constant__ TcGemmArgs g)
 {
   extern __shared__ uint8_t smem_raw[];
@@ -355,9 +360,13 @@ __global__ void __launch_bounds__(128) k_tc_gemm(const __grid_constant__ TcGemmA
     // Regions of the stages' memory, free now.  FP32 (result, old result): 4
     // boxes of 32 columns, 64 KiB; BF16: 2 boxes of 64 columns, 32 KiB: the
     // result in the first half, or past the stages beside an FP32 result; the
-    // matrix that is read in the second half.
-    uint8_t *r32 = smem, *e16 = smem + kTcM * kTcN * 2;
-    uint8_t *r16 = g.c32 ? smem + kStages * 2 * kTcTileBytes : smem;
+    // matrix that is read in the second half (a row's FP32 result overwrites
+    // there what its thread has used), or past the stages where the old result
+    // arrives in both halves (a BF16 result then takes its place column by
+    // column, as it is used).
+    uint8_t *past = smem + kStages * 2 * kTcTileBytes;
+    uint8_t *r32 = smem, *e16 = kBoth && g.accumulate ? past : smem + kTcM * kTcN * 2;
+    uint8_t *r16 = g.c32 ? past : smem;
     const bool reads16 = g.masked || g.residual;
     if (reads16 || g.accumulate) {
       if (tid == 0) {
@@ -412,6 +421,12 @@ __global__ void __launch_bounds__(128) k_tc_gemm(const __grid_constant__ TcGemmA
 #pragma unroll
           for (int j = 0; j < 32; j++)
             if (!(e[j] > 0.0f)) v[j] = 0.0f;
+        }
+        if (kBoth && g.mask && row < g.M) {
+          const __nv_bfloat16 *mk = g.mask + (size_t)row * g.ldm + n0 + c0;
+#pragma unroll
+          for (int j = 0; j < 32; j++)
+            if (!(__bfloat162float(mk[j]) > 0.0f)) v[j] = 0.0f;
         }
         if (g.partials) {
           if (row < g.M) {
@@ -515,14 +530,15 @@ uph_status launch_tc_gemm(const GemmCall &c, cudaStream_t s)
     return fail(UPH_BAD_ARG, "tc_gemm: split-K writes a dense FP32 result only, without bias, ReLU or mask");
   if (splits == 1 && !c.c_f32 && !c.c_bf16) return fail(UPH_BAD_ARG, "tc_gemm: no output");
   if (splits == 1 && c.accumulate && !c.c_f32) return fail(UPH_BAD_ARG, "tc_gemm: accumulate needs c_f32");
-  if (c.mask && c.residual) return fail(UPH_BAD_ARG, "tc_gemm: a mask or a residual, not both");
   if (c.col_sums && (!c.a_trans || splits <= 1 || !c.col_partials || c.M % 4))
     return fail(UPH_BAD_ARG, "tc_gemm: column sums go with a split-K product of a transposed A");
   static bool configured = false;
   if (!configured) {
-    UPH_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcRowStages>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    UPH_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcRowStages, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   tc_smem_bytes(kTcRowStages, true)));
-    UPH_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcSplitStages>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    UPH_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcRowStages, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  tc_smem_bytes(kTcRowStages, true)));
+    UPH_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcSplitStages, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   tc_smem_bytes(kTcSplitStages, false)));
     configured = true;
   }
@@ -545,7 +561,9 @@ uph_status launch_tc_gemm(const GemmCall &c, cudaStream_t s)
   splits = (c.K + kps - 1) / kps;
   g.bias = c.bias;
   g.relu = c.relu;
-  g.masked = c.mask != nullptr;
+  g.masked = c.mask && !c.residual;
+  g.mask = c.residual ? (const __nv_bfloat16 *)c.mask : nullptr;
+  g.ldm = c.ldm;
   g.residual = c.residual != nullptr;
   g.accumulate = splits > 1 ? 0 : c.accumulate;
   // split-K partials leave by TMA where a split's tiles are whole boxes
@@ -560,17 +578,20 @@ uph_status launch_tc_gemm(const GemmCall &c, cudaStream_t s)
     if (tr != UPH_OK) return tr;
   }
   if (g.c16) tr = make_tensor_map(&g.tm_c16, c.c_bf16, c.M, c.N, ldc16 * 2, kTcM);
-  if (tr == UPH_OK && c.mask) tr = make_tensor_map(&g.tm_e16, c.mask, c.M, c.N, c.ldm * 2, kTcM);
+  if (tr == UPH_OK && g.masked) tr = make_tensor_map(&g.tm_e16, c.mask, c.M, c.N, c.ldm * 2, kTcM);
   if (tr == UPH_OK && c.residual) tr = make_tensor_map(&g.tm_e16, c.residual, c.M, c.N, c.ldr * 2, kTcM);
   if (tr != UPH_OK) return tr;
+  const bool both = (c.mask && c.residual) || (g.accumulate && (c.mask || c.residual));
   g.col_partials = splits > 1 && c.col_sums ? c.col_partials : nullptr;
   g.err = c.err;
   g.stall = c.stall;
   dim3 grid((c.M + kTcM - 1) / kTcM, c.N / kTcN, splits);
   if (splits > 1)
-    k_tc_gemm<kTcSplitStages><<<grid, 128, tc_smem_bytes(kTcSplitStages, false), s>>>(g);
+    k_tc_gemm<kTcSplitStages, false><<<grid, 128, tc_smem_bytes(kTcSplitStages, false), s>>>(g);
+  else if (both)
+    k_tc_gemm<kTcRowStages, true><<<grid, 128, tc_smem_bytes(kTcRowStages, true), s>>>(g);
   else
-    k_tc_gemm<kTcRowStages><<<grid, 128, tc_smem_bytes(kTcRowStages, g.c32 && g.c16), s>>>(g);
+    k_tc_gemm<kTcRowStages, false><<<grid, 128, tc_smem_bytes(kTcRowStages, g.c32 && g.c16), s>>>(g);
   if (splits > 1) {
     const int count = c.M * c.N, cols = c.col_sums ? c.M : 0;
     const int blocks = (count / 4 + 31) / 32 + (cols / 4 + 31) / 32;
@@ -609,6 +630,35 @@ extern "C" uph_status uph_tc_gemm_bf16(const void *A, int32_t lda, const void *B
   c.splits = splits;
   c.partials = partials;
   c.accumulate = accumulate;
+  c.err = err;
+  return launch_tc_gemm(c, (cudaStream_t)stream);
+}
+
+// C ABI for tests: a row product with the whole epilogue (GemmCall); mask and
+// residual are BF16 [M x ldc] or null.
+extern "C" uph_status uph_tc_gemm_bf16_epilogue(const void *A, int32_t lda, const void *B, int32_t ldb, int32_t M,
+                                                int32_t N, int32_t K, const float *bias, const void *residual,
+                                                int32_t accumulate, int32_t relu, const void *mask, float *c_f32,
+                                                void *c_bf16, int32_t ldc, unsigned *err, void *stream)
+{
+  GemmCall c;
+  c.A = A;
+  c.lda = lda;
+  c.B = B;
+  c.ldb = ldb;
+  c.M = M;
+  c.N = N;
+  c.K = K;
+  c.bias = bias;
+  c.residual = residual;
+  c.ldr = ldc;
+  c.accumulate = accumulate;
+  c.relu = relu;
+  c.mask = mask;
+  c.ldm = ldc;
+  c.c_f32 = c_f32;
+  c.c_bf16 = c_bf16;
+  c.ldc = ldc;
   c.err = err;
   return launch_tc_gemm(c, (cudaStream_t)stream);
 }
