@@ -73,6 +73,11 @@ struct RefAcc {
   double drho_a, dpa_v, dpa_d, ax_a, ay_a;
   double frho, fp, fu, fv;
 };
+__device__ __forceinline__ bool all_finite(const RefAcc &A)
+{
+  return isfinite((((A.drho + A.dpd) + (A.ax + A.ay)) + ((A.drho_a + A.dpa_v) + (A.dpa_d + A.ax_a))) +
+                  (((A.ay_a + A.frho) + (A.fp + A.fu)) + A.fv));
+}
 // the rates of one particle
 struct RefRates {
   double drho, dp, ax, ay;
@@ -196,7 +201,8 @@ __device__ __forceinline__ RefOwn make_own(const DevParams &P, const RefRec &r)
 // About 105 FP64 operations.
 // wall: the pair's wall force acts (i side fluid, partner a wall).
 // kMasked: a pair that is not `on` contributes zeros (both kernels hold a
-// power of t as a factor) instead of being branched around.
+// power of t as a factor) instead of being branched around; zero times a
+// partner's field is zero only if the field is finite (RefStream::particle).
 template <bool kMasked>
 __device__ __forceinline__ void ref_pair(const DevParams &P, const RefOwn &a, const RefRec &b, double dxa, double dya,
                                          double r2, bool isI, bool on, bool wall, RefAcc &A)
@@ -746,6 +752,23 @@ struct RefStream {
       const bool isI = (c & kCandI) != 0u;
       my_pairs += on && isI;
       ref_pair<true>(P, o, b, dxa, dya, r2, isI, on, on && (c & kCandWall), A);
+    }
+    // A candidate outside the radius, or an excluded one, added zero times its
+    // fields: not zero where one of them is not finite.  Then the pairs alone
+    // are summed again.  (Branching around such candidates in the loop above
+    // costs every step 1.2 to 1.8 %: 500,000 particles 211 -> 215 us.)
+    if (__builtin_expect(!all_finite(A), 0)) {
+      A = RefAcc{};
+      CandReader<kLanes> again;
+      const int m = again.init(stream.G, P.nf, a);
+      for (int e = 0; e < m; e++) {
+        const unsigned c = again.next(e);
+        const RefRec &b = r[c & kCandRec];
+        const double dxa = o.r.x - b.x, dya = o.r.y - b.y;
+        const double r2 = exact_r2(dxa, dya);
+        if (r2 < P.r2cut && r2 > DBL_EPSILON && !(c & kCandNoPair))
+          ref_pair<false>(P, o, b, dxa, dya, r2, (c & kCandI) != 0u, true, (c & kCandWall) != 0u, A);
+      }
     }
     stream.done_reading();
     if constexpr (kLanes > 1) {

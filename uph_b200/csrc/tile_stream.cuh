@@ -16,7 +16,8 @@
 //
 // Every candidate is put through the exact pair test inside the pair loop;
 // one that fails is summed with a zero kernel, so a warp's lanes stay
-// together and no listing is needed.  Partners are visited in the candidate
+// together and no listing is needed.  (Where that gives a sum that is not
+// finite, the particle's pairs are summed again without the others.)  Partners are visited in the candidate
 // list's order, the stencil walk's, so with one lane per particle the sums
 // are those of the other passes.
 //

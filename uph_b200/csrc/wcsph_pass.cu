@@ -126,7 +126,9 @@ struct WcAcc {
 
 // the sums of one pair (a, b), a = the own particle
 // (the wall forces apart).  kMasked: a pair that is not `on` contributes
-// zeros (its kernel gradient is zero) instead of being branched around.
+// zeros (its kernel gradient is zero) instead of being branched around; zero
+// times a partner's field is zero only if the field is finite
+// (WcStream::particle).
 template <bool kMasked, typename Real, typename Rec>
 __device__ __forceinline__ void wc_pair(const DevParams &P, const Rec &a, const Rec &b, bool on, Real &drho, Real &ax,
                                         Real &ay)
@@ -606,6 +608,25 @@ struct WcStream {
       else
         wc_pair<true, Real>(P, own, d, on, drho, ax, ay);
       if (on && (c & kCandWall)) wc_wall(P, own, d, W);
+    }
+    // as in the REF pass: what a candidate that is no pair added is not zero
+    // where a field of it is not finite (3.7 % of a step of 2,000,000 FP32
+    // particles where the loop above branches instead)
+    if (__builtin_expect(!isfinite(drho + ax + ay), 0)) {
+      drho = ax = ay = 0;
+      CandReader<kLanes> again;
+      const int m = again.init(stream.G, P.nf, a);
+      for (int e = 0; e < m; e++) {
+        const unsigned c = again.next(e);
+        const unsigned char *p = buf + (size_t)(c & kCandRec) * kStride;
+        const WcRaw &d = *reinterpret_cast<const WcRaw *>(p);
+        const double r2 = exact_r2(own.x - d.x, own.y - d.y);
+        if (!(r2 < P.r2cut && r2 > DBL_EPSILON) || (c & kCandNoPair)) continue;
+        if constexpr (kF32)
+          wc_pair<false, Real>(P, of, *reinterpret_cast<const WcPair32 *>(p + sizeof(WcRaw)), true, drho, ax, ay);
+        else
+          wc_pair<false, Real>(P, own, d, true, drho, ax, ay);
+      }
     }
     stream.done_reading();
     if constexpr (kLanes > 1) {
