@@ -218,7 +218,7 @@ uph_status uph_sim_set_fused_step(uph_sim *sim, int32_t enable);
  * particles can close before the next build (up to 32 of them at h = 1.3 dx,
  * more for wider kernels), and the passes until the next build test only
  * those.  With 0 every step lists them afresh from the cell stencil.  The
- * pairs, their order and so the results are bit-identical either way.  (The
+ * lists, the pairs, their order and so the results are bit-identical either way.  (The
  * reference rebuilds its kd-tree search every call, Search.cc:5-44.) */
 uph_status uph_sim_set_candidate_lists(uph_sim *sim, int32_t enable);
 

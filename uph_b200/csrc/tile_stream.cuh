@@ -328,7 +328,12 @@ constexpr size_t kRecordSmemBytes = sizeof(RecordRing) + sizeof(RecordSmem) * (k
 // overflowed, no room in the stream's arrays) goes onto the list of hard
 // tiles.  Only FP32 distances are computed: a candidate within the list
 // radius (F32Test::vl, rounding included) is listed, and the pair loop
-// decides.
+// decides.  The distances are those of the positions the list binned
+// (DevParams::xbin), which the skin bounds the motion from: a pass that
+// records later than it was built (walls may have moved meanwhile) writes the
+// same lists, as does one that records at every launch, so which lanes and
+// which tiles a pair falls to, and with them every rounding, do not depend on
+// when lists are written.
 template <bool kBrute, int kGroup>
 __device__ __forceinline__ void stream_record(const DevParams &P, const SlotArrays &S, const CellGrid &G, int tile,
                                               RecordSmem &R, RecordRing &ring)
@@ -408,8 +413,8 @@ __device__ __forceinline__ void stream_record(const DevParams &P, const SlotArra
       }
 #pragma unroll
       for (int u = 0; u < kU; u++) {
-        x[u] = S.x[s[u]];
-        y[u] = S.y[s[u]];
+        x[u] = P.xbin[s[u]];
+        y[u] = P.ybin[s[u]];
         const int o = S.orig[s[u]];
         who[u] = (unsigned)o | (S.itype[s[u]] >= 2 ? kWhoWall : 0u) | (o >= P.b0 && o < P.b1 ? kWhoBoundary : 0u);
       }
