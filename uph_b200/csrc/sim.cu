@@ -462,6 +462,22 @@ uph_status check_error_word(uph_sim *s)
   return UPH_OK;
 }
 
+// Whether a lattice's tiles fit the stream (tile_stream.cuh): the block's
+// records a buffer, the core's particles a CTA's threads.  Where they do not
+// (wide kernels, h > 1.9 dx at the default tiles; large tiles), the step would
+// take every tile as a hard one, two at a time per SM and each block's in a
+// fixed order; the tiled pass behind a list launch of its own is faster.  us a
+// step, hard tiles / tiled pass: nearNeighbor 61, REF, 40,000 particles 168 /
+// 113; 91, 200,000 particles, REF 600 / 509, FP32 890 / 635; tile 16 and reach 1
+// at h = 1.3 dx, REF, 61,000 481 / 380.  A block that just fits streams: 45 (478
+// records), REF, 200,000 254, against 287 with the next smaller tile.
+bool tiles_stream(const DevParams &P)
+{
+  if (!(P.dx > 0)) return true;
+  const double per_cell = (P.cell / P.dx) * (P.cell / P.dx), edge = P.tile + 2 * P.reach;
+  return edge * edge * per_cell <= kStreamCap && (double)P.tile * P.tile * per_cell * P.lanes <= kTileThreads;
+}
+
 // what follows the rate pass of an evaluation
 uph_status after_pass(uph_sim *s)
 {
@@ -491,7 +507,7 @@ uph_status rate_pass(uph_sim *s, bool refresh, bool step = false, const StepOut 
   // the steps of uph_sim_step: one launch, the cell list in it (a lone
   // evaluation, after an upload that rebuilt the list, would only write
   // candidate lists nobody reads)
-  if (step && s->P.knn == 0 && s->P.nf > 0 &&
+  if (step && s->P.knn == 0 && s->P.nf > 0 && tiles_stream(s->P) &&
       (s->P.profile != UPH_PROFILE_REF || s->P.flag_init_simul == 1)) {
     Timer t(s, KF_PASS);
     const StepArgs A{PassStats{s->d_niac + 1, s->d_max_nb + 1}, st, s->d_step_done, s->d_moved, s->d_ticket, s->d_phases,
