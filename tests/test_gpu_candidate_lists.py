@@ -82,3 +82,20 @@ def test_kept_lists_change_no_bit(profile, precision, n, tile):
             assert s.stats()["list_builds"] > 2
     for f, a in got[0].items():
         assert np.array_equal(a, got[1][f]), f
+
+
+@pytest.mark.parametrize("precision,tile,launches", [(PREC_FP64, 11, 5), (PREC_FP32_PAIR, None, 5), (PREC_FP64, 7, 3)])
+def test_steps_without_kept_lists(precision, tile, launches):
+    """With one lane per particle nothing is recorded for one step alone: a
+    list launch and the tiled pass, behind the call's predictor."""
+    from uph_b200.sim import Simulation
+    d, st = _stirred(3000)
+    with Simulation(d.uph_params(profile=PROFILE_WCSPH, precision=precision)) as s:
+        if tile:
+            s.set_tuning(2, tile, 64)
+        s.set_candidate_lists(False)
+        s.upload(st, 0)
+        s.step(1)
+        before = s.launch_count()
+        s.step(2)
+        assert s.launch_count() - before == launches
