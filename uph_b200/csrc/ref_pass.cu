@@ -866,14 +866,11 @@ __device__ __forceinline__ void knn_walk(const DevParams &P, const CellGrid &G, 
   }
 }
 
-__global__ void __launch_bounds__(256) k_knn_cut(const DevParams P, const SlotArrays S, const CellGrid G,
-                                                 const VirtualPoints V)
+// the cut of query a, by a warp
+__device__ __forceinline__ void knn_cut_query(const DevParams &P, const SlotArrays &S, const CellGrid &G,
+                                              const VirtualPoints &V, int a, KnnSmem &M)
 {
-  __shared__ KnnSmem smem[8];
   const int lane = threadIdx.x & 31;
-  const int a = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (a >= P.nf) return;
-  KnnSmem &M = smem[threadIdx.x >> 5];
   const double xa = S.x[a], ya = S.y[a];
   const int cell = G.cell_of[a];
   // the virtual mirror particles are points of the reference's search too
@@ -1019,11 +1016,73 @@ __global__ void __launch_bounds__(256) k_knn_cut(const DevParams P, const SlotAr
   }
 }
 
-void launch_knn_cut(const DevParams &P, const SlotArrays &S, const CellGrid &G, const VirtualPoints &V,
+// points of one grid in radius of a query, by a thread
+__device__ __forceinline__ int knn_count(const DevParams &P, const CellGrid &G, const double *x, const double *y,
+                                         int cell, double xa, double ya, int self)
+{
+  NeighbourCursor cur;
+  cur.init(P, G, cell);
+  int n = 0, pos = 0;
+  for (int m = cur.next_batch<4>(pos); m > 0; m = cur.next_batch<4>(pos)) {
+    int b[4];
+    double r2[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) b[u] = G.list[pos + (u < m ? u : 0)];
+#pragma unroll
+    for (int u = 0; u < 4; u++) r2[u] = exact_r2(xa - x[b[u]], ya - y[b[u]]);
+#pragma unroll
+    for (int u = 0; u < 4; u++) n += u < m && b[u] != self && r2[u] < P.r2cut && r2[u] > DBL_EPSILON;
+  }
+  return n;
+}
+
+// kCount: a warp's lanes first count the points in radius of a query each and
+// the warp goes on with those of more than knn points only, one after the
+// other.  For a lattice of at most knn points in radius (`few` of
+// launch_knn_cut): where the cap hardly cuts, a warp for every query is mostly
+// idle lanes.  10 steps of 100,000 particles at h = 1.3 dx (21 in radius) under
+// the cap of 40: 983 us, 1,600 with a warp each; of 40,000 in motion, 25 in
+// radius 722 against 925, 37 884 / 1,055, 40 1,032 / 1,096; from 45 on, where a
+// warp each takes 1,255, most queries are cut.
+template <bool kCount>
+__global__ void __launch_bounds__(256) k_knn_cut(const DevParams P, const SlotArrays S, const CellGrid G,
+                                                 const VirtualPoints V)
+{
+  __shared__ KnnSmem smem[8];
+  const int lane = threadIdx.x & 31;
+  const int w = blockIdx.x * 8 + (threadIdx.x >> 5);
+  KnnSmem &M = smem[threadIdx.x >> 5];
+  if constexpr (!kCount) {
+    if (w < P.nf) knn_cut_query(P, S, G, V, w, M);
+  } else {
+    const int a = 32 * w + lane;
+    bool more = false;
+    if (a < P.nf) {
+      const double xa = S.x[a], ya = S.y[a];
+      const int cell = G.cell_of[a];
+      int n = knn_count(P, G, S.x, S.y, cell, xa, ya, a);
+      if (V.grid.list) n += knn_count(P, V.grid, V.x, V.y, cell, xa, ya, -1);
+      more = n > P.knn;
+      if (!more) {
+        P.kcut_d2[a] = __longlong_as_double(0x7ff0000000000000ll);  // +inf: nothing is cut
+        P.kcut_j[a] = INT_MAX;
+      }
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, more); m; m &= m - 1) {
+      knn_cut_query(P, S, G, V, 32 * w + __ffs(m) - 1, M);
+      __syncwarp();
+    }
+  }
+}
+
+void launch_knn_cut(const DevParams &P, const SlotArrays &S, const CellGrid &G, const VirtualPoints &V, bool few,
                     cudaStream_t s)
 {
   if (P.nf <= 0 || P.knn <= 0) return;
-  k_knn_cut<<<(P.nf + 7) / 8, 256, 0, s>>>(P, S, G, V);
+  if (few)
+    k_knn_cut<true><<<(P.nf + 255) / 256, 256, 0, s>>>(P, S, G, V);
+  else
+    k_knn_cut<false><<<(P.nf + 7) / 8, 256, 0, s>>>(P, S, G, V);
 }
 
 // ---- stressType 2 (ClassicShearStress, derivatives.c:1686-1721, and

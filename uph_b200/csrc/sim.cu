@@ -462,6 +462,13 @@ uph_status check_error_word(uph_sim *s)
   return UPH_OK;
 }
 
+// Whether a lattice has at most knn points in radius, so that the cap cuts few
+// queries (crowded ones).  (A search knows no lattice.)
+bool few_in_radius(const uph_sim *s)
+{
+  return !s->search_only && 3.14159 * s->P.r2cut <= s->P.knn * s->P.dx * s->P.dx;
+}
+
 // Whether a lattice's tiles fit the stream (tile_stream.cuh): the block's
 // records a buffer, the core's particles a CTA's threads.  Where they do not
 // (wide kernels, h > 1.9 dx at the default tiles; large tiles), the step would
@@ -542,7 +549,7 @@ uph_status rate_pass(uph_sim *s, bool refresh, bool step = false, const StepOut 
     }
   }
   if (s->P.knn > 0) {
-    launch_knn_cut(s->P, s->S, s->G, vp, s->stream);
+    launch_knn_cut(s->P, s->S, s->G, vp, few_in_radius(s), s->stream);
     s->launches++;
     s->kcut_fresh = true;
   }
@@ -1608,7 +1615,7 @@ extern "C" uph_status uph_sim_approx_vorticity(uph_sim *s, double *vorticity)
   if (s->P.knn > 0 && !s->kcut_fresh) {
     VirtualPoints vp = {nullptr, nullptr, CellGrid{}};
     if (s->P.nvrules > 0 && s->have_rates) vp = VirtualPoints{s->vb.x, s->vb.y, s->gv};
-    launch_knn_cut(s->P, s->S, s->G, vp, q);
+    launch_knn_cut(s->P, s->S, s->G, vp, few_in_radius(s), q);
     s->launches++;
     s->kcut_fresh = true;
   }
@@ -1634,7 +1641,7 @@ extern "C" uph_status uph_sim_pairs(uph_sim *s, int64_t cap, int32_t *i_pair, in
     // the virtual particles of the last evaluation, when the virtualType has them
     VirtualPoints vp = {nullptr, nullptr, CellGrid{}};
     if (s->P.nvrules > 0 && s->have_rates) vp = VirtualPoints{s->vb.x, s->vb.y, s->gv};
-    launch_knn_cut(s->P, s->S, s->G, vp, q);
+    launch_knn_cut(s->P, s->S, s->G, vp, few_in_radius(s), q);
     s->launches++;
     s->kcut_fresh = true;
   }

@@ -315,8 +315,8 @@ struct VirtualPoints {
   CellGrid grid;
 };
 // the knn cap's cut of every fluid query (P.kcut_*), from the cell list and
-// the virtual points
-void launch_knn_cut(const DevParams &P, const SlotArrays &S, const CellGrid &G, const VirtualPoints &V,
+// the virtual points; few: most queries have at most knn points in radius
+void launch_knn_cut(const DevParams &P, const SlotArrays &S, const CellGrid &G, const VirtualPoints &V, bool few,
                     cudaStream_t s);
 // Scratch and results of the virtual particles: flags and offsets by
 // (rule, reference fluid index), positions, source fluid index and rule of
