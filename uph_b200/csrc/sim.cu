@@ -462,6 +462,13 @@ uph_status check_error_word(uph_sim *s)
   return UPH_OK;
 }
 
+// Whether a simulation's steps stream recorded tiles at all (tile_stream.cuh):
+// not under the k-nearest cap and not in the particle-packing initialisation.
+bool steps_stream(const DevParams &P)
+{
+  return P.knn == 0 && P.nf > 0 && (P.profile != UPH_PROFILE_REF || P.flag_init_simul == 1);
+}
+
 // Whether a lattice has at most knn points in radius, so that the cap cuts few
 // queries (crowded ones).  (A search knows no lattice.)
 bool few_in_radius(const uph_sim *s)
@@ -517,8 +524,7 @@ uph_status rate_pass(uph_sim *s, bool refresh, bool step = false, const StepOut 
   // a step would record every tile for itself alone: the tiled pass is faster
   // (61,000 particles, REF 88 / 74 us a step, FP32 77 / 59; 300,000 alike) and
   // sums in the same order, unless a particle's pairs are dealt out to lanes.
-  if (step && s->P.knn == 0 && s->P.nf > 0 && tiles_stream(s->P) && (s->cand_lists || s->P.lanes > 1) &&
-      (s->P.profile != UPH_PROFILE_REF || s->P.flag_init_simul == 1)) {
+  if (step && steps_stream(s->P) && tiles_stream(s->P) && (s->cand_lists || s->P.lanes > 1)) {
     Timer t(s, KF_PASS);
     const StepArgs A{PassStats{s->d_niac + 1, s->d_max_nb + 1}, st, s->d_step_done, s->d_moved, s->d_ticket, s->d_phases,
                      s->cand_lists ? 0 : 1, s->d_itime};
@@ -612,7 +618,7 @@ cudaError_t alloc_grid(uph_sim *s)
   // about 225 of them; one beyond the capacity is handled as a hard tile
   const long long ntiles = (long long)s->P.ntx * (s->P.ncy / s->P.tile);
   const long long want = std::min(ntiles, (long long)s->P.nf / 64 + 1024);
-  if (!s->search_only && ntiles > s->stream_tiles) {
+  if (!s->search_only && steps_stream(s->P) && tiles_stream(s->P) && ntiles > s->stream_tiles) {
     StreamTiles &t = G.st;
     if (s->stream_block) cudaFree(s->stream_block);
     s->stream_block = nullptr;
@@ -838,10 +844,10 @@ DevParams make_dev_params(const uph_params *p)
   int tile = kCellTile;
   const double hdx = p->dx > 0 ? h / p->dx : 1.0;
   if (hdx > 1.4) tile = std::max(2, (int)floor(kCellTile * 1.3 / hdx));
-  if (p->n_fluid <= kTwoLanesMax && p->precision != UPH_PREC_FP32_PAIR && p->knn_cap == 0)
+  P.knn = p->knn_cap;
+  if (p->n_fluid <= kTwoLanesMax && p->precision != UPH_PREC_FP32_PAIR && steps_stream(P))
     tile = std::max(2, tile * (p->n_fluid <= kFourLanesMax ? 5 : 7) / kCellTile);
   set_grid_geometry(P, kCellReach, tile);
-  P.knn = p->knn_cap;
   P.kcut_d2 = nullptr;
   P.kcut_j = nullptr;
   P.str_xx = P.str_xy = P.str_yy = nullptr;
@@ -924,14 +930,16 @@ uph_status create_sim(const uph_params *p, uph_sim **out, bool search_only)
       B.want(&s->P.str_yy, (size_t)n);
     }
     B.want(&mass0, 1);
-    // room for 1.3 times the candidates of a lattice (pi (R_l / dx)^2, R_l
-    // the list radius), so that moving water seldom overflows: 32 entries at
-    // h = 1.3 dx
-    const double Rl = sqrt(s->P.r2cut) + 2.0 * 1.4142135623730951 * s->P.skin;
-    const double want = 1.3 * 3.14159 * (Rl / p->dx) * (Rl / p->dx);
-    G.vl_cap = want >= kVlCapMax ? kVlCapMax : std::max(16, (int)ceil(want / 8.0) * 8);
-    B.want(&G.vl, (size_t)nf * G.vl_cap);
-    B.want(&G.vl_n, (size_t)nf);
+    if (steps_stream(s->P)) {
+      // room for 1.3 times the candidates of a lattice (pi (R_l / dx)^2, R_l
+      // the list radius), so that moving water seldom overflows: 32 entries at
+      // h = 1.3 dx
+      const double Rl = sqrt(s->P.r2cut) + 2.0 * 1.4142135623730951 * s->P.skin;
+      const double want = 1.3 * 3.14159 * (Rl / p->dx) * (Rl / p->dx);
+      G.vl_cap = want >= kVlCapMax ? kVlCapMax : std::max(16, (int)ceil(want / 8.0) * 8);
+      B.want(&G.vl, (size_t)nf * G.vl_cap);
+      B.want(&G.vl_n, (size_t)nf);
+    }
     if (s->P.nvrules > 0) {
       V.cap = s->P.nvrules * nf;
       B.want(&V.flags, (size_t)V.cap);
