@@ -229,8 +229,11 @@ uph_status uph_sim_set_candidate_lists(uph_sim *sim, int32_t enable);
 uph_status uph_sim_set_tuning(uph_sim *sim, int32_t reach, int32_t tile, int32_t reorder_interval);
 
 /* Picks the tuning by timing `trial_steps` steps per candidate on this
- * simulation (a coordinate search over reach, tile and interval; it advances
- * the simulation by about 9 (trial_steps + 2) steps) and applies the fastest.
+ * simulation (a coordinate search over reach, tile and interval from the
+ * simulation's defaults; it advances the simulation by up to 9 (trial_steps +
+ * 2) steps) and applies the fastest, where that is 5 % faster than the
+ * defaults.  An interval other than the default's is tried only if trial_steps
+ * is at least as long.
  * Results are cached per size class, so later sims of the same class are
  * tuned without trials.  choice[3] receives (reach, tile, interval);
  * *ms_per_step the best trial's time (0 when taken from the cache). */

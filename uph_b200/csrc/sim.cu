@@ -710,6 +710,24 @@ void set_grid_geometry(DevParams &P, int reach, int tile)
     P.lanes = core * 4 <= kTileThreads ? 4 : core * 2 <= kTileThreads ? 2 : 1;
 }
 
+// The default tile at the default reach.  Cells of half the search radius: a 5
+// x 5 block holds 25 h^2 of candidates against 36 h^2 for a 3 x 3 block of
+// radius-wide cells.  A cell then holds about ((1 + skin) h / dx)^2 particles
+// of a lattice; the tile of one lane per particle (11 cells at h = 1.3 dx)
+// shrinks for wider kernels so that its particles fit one round of a CTA and
+// its block the tiled passes' shared-memory records.
+int one_lane_tile(const DevParams &P)
+{
+  const double hdx = P.dx > 0 ? P.h / P.dx : 1.0;
+  return hdx > 1.4 ? std::max(2, (int)floor(kCellTile * 1.3 / hdx)) : kCellTile;
+}
+int default_tile(const DevParams &P)
+{
+  const int tile = one_lane_tile(P);
+  if (P.nf > kTwoLanesMax || P.precision == UPH_PREC_FP32_PAIR || !steps_stream(P)) return tile;
+  return std::max(2, tile * (P.nf <= kFourLanesMax ? 5 : 7) / kCellTile);
+}
+
 // The mirror rules of each virtualType, in the reference's loop order
 // (derivatives.c:3195-4189).  Type 2's loops are commented out in the
 // reference; other types have none.
@@ -835,19 +853,8 @@ DevParams make_dev_params(const uph_params *p)
     P.hi_x += pad;
     P.hi_y += pad;
   }
-  // cells of half the search radius: a 5 x 5 block holds 25 h^2 of candidates
-  // against 36 h^2 for a 3 x 3 block of radius-wide cells.  A cell then holds
-  // about ((1 + skin) h / dx)^2 particles of a lattice; the default tile (11
-  // cells at h = 1.3 dx) shrinks for wider kernels so that a tile's
-  // particles fit one round of a CTA and its block the tiled passes'
-  // shared-memory records.
-  int tile = kCellTile;
-  const double hdx = p->dx > 0 ? h / p->dx : 1.0;
-  if (hdx > 1.4) tile = std::max(2, (int)floor(kCellTile * 1.3 / hdx));
   P.knn = p->knn_cap;
-  if (p->n_fluid <= kTwoLanesMax && p->precision != UPH_PREC_FP32_PAIR && steps_stream(P))
-    tile = std::max(2, tile * (p->n_fluid <= kFourLanesMax ? 5 : 7) / kCellTile);
-  set_grid_geometry(P, kCellReach, tile);
+  set_grid_geometry(P, kCellReach, default_tile(P));
   P.kcut_d2 = nullptr;
   P.kcut_j = nullptr;
   P.str_xx = P.str_xy = P.str_yy = nullptr;
@@ -1913,18 +1920,21 @@ extern "C" uph_status uph_sim_set_tuning(uph_sim *s, int32_t reach, int32_t tile
 namespace {
 
 struct TuneKey {
-  int profile, precision, nf_class, cell_class;
+  int profile, precision, nf_class, cell_class, tile;
   bool operator<(const TuneKey &o) const
   {
     if (profile != o.profile) return profile < o.profile;
     if (precision != o.precision) return precision < o.precision;
     if (nf_class != o.nf_class) return nf_class < o.nf_class;
-    return cell_class < o.cell_class;
+    if (cell_class != o.cell_class) return cell_class < o.cell_class;
+    return tile < o.tile;
   }
 };
 
 std::mutex g_tune_mutex;
 std::map<TuneKey, std::array<int, 3>> g_tune_cache;
+
+constexpr double kTuneGain = 0.95;
 
 int log2_class(double v) { return v < 1.0 ? 0 : (int)floor(log2(v)); }
 
@@ -1951,21 +1961,26 @@ uph_status time_steps(uph_sim *s, int steps, double *ms)
 
 }  // namespace
 
-// Coordinate search over (cell reach, storage tile, re-sort interval): the
-// reach first with tile 11 and interval 64, then the tile at the best reach,
-// then the interval.  Each trial times `trial_steps` steps of this very
-// simulation, so tuning advances it by about 9 (trial_steps + 2) steps.
+// Coordinate search over (cell reach, storage tile, re-sort interval) from the
+// simulation's defaults: the reach first, then the tile at the best reach (two
+// cells less and more), then the interval.  Each trial times `trial_steps` steps of this very simulation, so
+// tuning advances it by up to 9 (trial_steps + 2) steps.  What a short trial
+// does not show must not decide: an interval is tried only where a trial is
+// long enough to hold a re-sort, and a choice has to win by kTuneGain, since a
+// trial's steps follow a list build and seldom hold one (12,000 particles, tile
+// 7 against 5: trials 19.4 to 20.2 / 20.0 us a step, a long run 23.1 / 19.2).
 // Results are cached per size class (profile, precision, log2 of the fluid
-// count, log2 of the radius-wide cell count); a sim of a cached class is set
-// without trials.
+// count, log2 of the radius-wide cell count, default tile); a sim of a cached
+// class is set without trials.
 extern "C" uph_status uph_sim_autotune(uph_sim *s, int32_t trial_steps, int32_t choice[3], double *ms_per_step)
 {
   if (!s || !choice) return fail(UPH_BAD_ARG, "uph_sim_autotune: NULL argument");
   if (trial_steps < 1) return fail(UPH_BAD_ARG, "uph_sim_autotune: trial_steps must be positive");
   DevParams P1 = s->P;
   set_grid_geometry(P1, 1, 1);
-  const TuneKey key{s->P.profile, s->P.precision, log2_class(s->P.nf), log2_class((double)P1.ncx * P1.ncy)};
-  std::array<int, 3> best{kCellReach, kCellTile, kReorderInterval};
+  const int tile0 = default_tile(s->P);
+  const TuneKey key{s->P.profile, s->P.precision, log2_class(s->P.nf), log2_class((double)P1.ncx * P1.ncy), tile0};
+  std::array<int, 3> best{kCellReach, tile0, kReorderInterval};
   bool cached = false;
   {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
@@ -1982,23 +1997,37 @@ extern "C" uph_status uph_sim_autotune(uph_sim *s, int32_t trial_steps, int32_t 
       if (r != UPH_OK) return r;
       return time_steps(s, trial_steps, ms);
     };
-    best_ms = 1e300;
+    // the defaults twice: the first trial may find the GPU at its idle clocks
+    for (int k = 0; k < 2; k++) {
+      uph_status r = trial(best, &best_ms);
+      if (r != UPH_OK) return r;
+    }
     for (int axis = 0; axis < 3; axis++) {
-      static const int options[3][3] = {{1, 2, 3}, {9, 11, 13}, {16, 64, 256}};
-      std::array<int, 3> axis_best = best;
-      for (int v : options[axis]) {
-        std::array<int, 3> c = best;
-        c[axis] = v;
+      std::vector<std::array<int, 3>> options;
+      if (axis == 0) {
+        options = {{1, tile0, best[2]}, {3, tile0, best[2]}};
+        // (the tile of one lane at the default reach, of several at this one)
+        if (one_lane_tile(s->P) != tile0) options.push_back({3, one_lane_tile(s->P), best[2]});
+      } else if (axis == 1) {
+        options = {{best[0], best[1] - 2, best[2]}, {best[0], best[1] + 2, best[2]}};
+      } else {
+        for (int v : {16, 256})
+          if (v <= trial_steps) options.push_back({best[0], best[1], v});
+      }
+      double axis_ms = kTuneGain * best_ms;
+      bool better = false;
+      for (const std::array<int, 3> &c : options) {
         double ms = 0.0;
         uph_status r = trial(c, &ms);
         if (r == UPH_BAD_ARG) continue;  // e.g. a grid too large for this reach
         if (r != UPH_OK) return r;
-        if (ms < best_ms) {
-          best_ms = ms;
-          axis_best = c;
+        if (ms < axis_ms) {
+          axis_ms = ms;
+          best = c;
+          better = true;
         }
       }
-      best = axis_best;
+      if (better) best_ms = axis_ms;
     }
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     g_tune_cache[key] = best;
