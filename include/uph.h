@@ -227,6 +227,9 @@ uph_status uph_sim_set_candidate_lists(uph_sim *sim, int32_t enable);
  * 2 reach <= 32) and the storage re-sort interval in steps.  Defaults 2, 11
  * (5 and 7 for tanks of up to 15,000 and 30,000 particles in FP64), 64. */
 uph_status uph_sim_set_tuning(uph_sim *sim, int32_t reach, int32_t tile, int32_t reorder_interval);
+/* The tuning in force: tuning[4] receives reach, tile, interval and the lanes
+ * that share a particle's pairs in a step's pass (1, 2 or 4, from the tile). */
+uph_status uph_sim_get_tuning(const uph_sim *sim, int32_t tuning[4]);
 
 /* Picks the tuning by timing `trial_steps` steps per candidate on this
  * simulation (a coordinate search over reach, tile and interval from the

@@ -1917,6 +1917,16 @@ extern "C" uph_status uph_sim_set_tuning(uph_sim *s, int32_t reach, int32_t tile
   return reorder_fluid(s);
 }
 
+extern "C" uph_status uph_sim_get_tuning(const uph_sim *s, int32_t tuning[4])
+{
+  if (!s || !tuning) return fail(UPH_BAD_ARG, "uph_sim_get_tuning: NULL argument");
+  tuning[0] = s->P.reach;
+  tuning[1] = s->P.tile;
+  tuning[2] = s->reorder_interval;
+  tuning[3] = s->P.lanes;
+  return UPH_OK;
+}
+
 namespace {
 
 struct TuneKey {

@@ -112,6 +112,12 @@ class Simulation:
     def set_tuning(self, reach: int, tile: int, reorder_interval: int) -> None:
         _lib.check(self.lib.uph_sim_set_tuning(self.handle, reach, tile, reorder_interval), "uph_sim_set_tuning")
 
+    def tuning(self):
+        """(reach, tile, interval, lanes per particle) in force."""
+        t = (C.c_int32 * 4)()
+        _lib.check(self.lib.uph_sim_get_tuning(self.handle, t), "uph_sim_get_tuning")
+        return tuple(t)
+
     def autotune(self, trial_steps: int = 10):
         """Native autotuner; returns ((reach, tile, interval), best ms/step or 0 if cached)."""
         choice = (C.c_int32 * 3)()
