@@ -99,3 +99,31 @@ def test_steps_without_kept_lists(precision, tile, launches):
         before = s.launch_count()
         s.step(2)
         assert s.launch_count() - before == launches
+
+
+@pytest.mark.parametrize("profile,precision", [(PROFILE_REF, PREC_FP64), (PROFILE_WCSPH, PREC_FP64),
+                                               (PROFILE_WCSPH, PREC_FP32_PAIR)])
+@pytest.mark.parametrize("piston_layers", [1, 3])
+def test_moving_walls_step_alike(profile, precision, piston_layers):
+    """A wave flume's piston (the reference's law, and a table) where steps
+    stream and where they take the tiled pass, as single calls and as a graph."""
+    from uph_b200.sim import Simulation
+    d = D.wave_flume(2.0, 0.4, 0.016, piston_layers=piston_layers, hydrostatic_walls=True)
+    st = d.initial_state()
+    got = []
+    for lists, graph in ((True, 0), (False, 0), (True, 30), (False, 30)):
+        with Simulation(d.uph_params(profile=profile, precision=precision)) as s:
+            s.set_tuning(2, 11, 64)
+            if d.wall_table is not None:
+                s.set_wall_motion(*d.wall_table)
+            s.set_candidate_lists(lists)
+            s.set_graph(graph)
+            s.upload(st, 0)
+            s.step(1)
+            s.step(30)
+            s.step(30)
+            got.append(s.download())
+    assert np.abs(got[0]["Position"] - st["Position"])[d.n_fluid:].max() > 0
+    for other in got[1:]:
+        for f, a in got[0].items():
+            assert np.array_equal(a, other[f]), f
