@@ -61,8 +61,8 @@ void launch_predict(const DevParams &P, const SlotArrays &S, cudaStream_t s)
 // runs right after.  Flags non-finite results.
 // The corrector of the fluid slots; with predict_next also the next step's
 // predictor, and with walls_next the next step's wall motion on the threads
-// past the fluid (its time from the device step counter, which the next
-// step's cell-list launch advances: (steps started + 1) dt).
+// past the fluid (its time from the device step counter, which this step has
+// advanced: (steps started + 1) dt).
 __global__ void k_correct(const DevParams P, const SlotArrays S, const WallTable W, int first_step, int predict_next,
                           int walls_next, unsigned *err, const int *d_itime)
 {

@@ -121,10 +121,10 @@ struct uph_sim {
   // next step starts the leapfrog afresh with the first-step half kick
   bool restart = false;
   int64_t serial = 0;  // distinct for every simulation this process creates
-  // the REF pass applies the leapfrog step (uph_sim_set_fused_step)
+  // the rate passes apply the leapfrog step (uph_sim_set_fused_step)
   bool fused_step = true;
-  // the tiled passes keep per-particle candidate lists between cell-list
-  // builds (uph_sim_set_candidate_lists)
+  // the steps keep candidate lists and recorded tiles between cell-list builds
+  // (uph_sim_set_candidate_lists)
   bool cand_lists = true;
   // per-evaluation diagnostics (off by default)
   bool diag_enabled = false;
@@ -1203,9 +1203,10 @@ bool walls_move(const uph_sim *s)
   return s->hp.n_moving > 0 && (s->W.enabled || ((mb == 1 || mb == 2 || mb == 3) && s->P.flag_init_simul == 1));
 }
 
-// Enqueues `nsteps` leapfrog steps on the sim's stream.  Where the rate pass
-// applies the step (StepOut) each step is the list launch and the pass, and
-// the two state buffers swap; else the pass and the corrector.  With
+// Enqueues `nsteps` leapfrog steps on the sim's stream.  A step's rate pass is
+// one launch that streams, or the list launch and the tiled pass (rate_pass).
+// Where the pass applies the step (StepOut) the two state buffers swap; else
+// the corrector follows.  With
 // `capturing` the sequence is being recorded into a CUDA graph: no host
 // synchronisation, no profiling events, and an even number of buffer swaps
 // (one more storage re-sort where needed) so the graph ends on the buffer it

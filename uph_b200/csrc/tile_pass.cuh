@@ -28,10 +28,10 @@ constexpr int kTileRowsMax = 32;   // rows and columns of a block (tile + 2 reac
 constexpr int kTileTabMax = (kTileRowsMax + 1) * kTileRowsMax;
 constexpr unsigned short kRoleI16 = 0x8000u;  // list-entry flag: this particle is the pair's i
 
-// one CTA's tile and block, in shared memory
 // a global line fetched into L2 ahead of its use
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// one CTA's tile and block, in shared memory
 struct TileBlock {
   int bx0, by0, W, H;          // block: first cell (x, y) and size in cells
   int ncore;                   // particles (of any kind) in the core cells
@@ -226,8 +226,9 @@ __device__ __forceinline__ F32Test make_f32_test(const DevParams &P, int cells, 
   const double R = sqrt(P.r2cut);
   const double E = (double)cells * P.cell;
   const double band = 32.0 * (E / R) * 0x1p-23 + 0x1p-20;
-  // between two builds a particle moves at most the skin along each axis,
-  // so a pair's distance shrinks by at most 2 sqrt(2) skin
+  // between two builds a particle moves at most the skin along each axis from
+  // where it was binned, so a pair's distance is at most 2 sqrt(2) skin less
+  // than it was there
   const double Rl = R + 2.0 * 1.4142135623730951 * P.skin;
   return F32Test{xa, ya, (float)(P.r2cut * (1.0 - band)), (float)(P.r2cut * (1.0 + band)),
                  (float)(P.r2cut * 1e-3), (float)(Rl * Rl * (1.0 + band))};

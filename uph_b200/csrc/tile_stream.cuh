@@ -24,11 +24,14 @@
 // What bounds it (500,000-particle tank, REF FP64): FP64 arithmetic, about
 // 105 operations per pair side, 46 M warp instructions or 79 us of the FP64
 // pipe, and beside it the pair loop's shared-memory reads (7.7 wavefronts
-// per 16-byte read, 72 us of that pipe) at 16 warps per SM.  Measured: the
+// per 16-byte read, 72 us of that pipe) at 16 warps per SM, 128 registers a
+// thread (k_ref_step, which holds the build, the recording and the hard tiles
+// too, spills 268 bytes of stores and 476 of loads, 424 and 592 in the
+// brute-force wall modes; k_wcsph_step none).  Measured: the
 // streaming step 0.168 ms in the kernel (0.229 for the pass that staged,
 // listed and summed one tile per CTA, plus 8 us for the list launch), the
 // recording step 0.285; us per step of 100-step calls, before and after:
-// REF 5,000 particles 44 and 26, 61,000 56 and 47, 500,000 253 and 190; WCSPH
+// REF 5,000 particles 44 and 22, 61,000 56 and 45, 500,000 253 and 190; WCSPH
 // FP64 300,000 in violent motion (a rebuild every third step) 198 and 142,
 // FP32 pairs 2,000,000 906 and 556.
 //

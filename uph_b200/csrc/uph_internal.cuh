@@ -213,13 +213,15 @@ struct CellGrid {
   int *rank;       // [n]
   int *totals;     // [kCellBuildMaxBlocks + 1]
   unsigned *bar;   // [kGridWords]
-  // The tiled passes' candidate lists and recorded tiles (the simulation's
-  // main grid only; null on other grids).  gen counts the builds that rebuilt
-  // the list; the recording pass after a build writes, for each fluid
-  // particle (by slot), vl_n candidates in vl (the layout of CandWriter): the
-  // records of its tile's block within the list radius (the search radius
-  // plus twice the largest displacement a rebuild allows), in the stencil
-  // walk's order, or vl_n == kVlOverflow when there were more than vl_cap.
+  // The candidate lists and recorded tiles of the steps that stream (the
+  // simulation's main grid only, and only where its steps stream; null
+  // elsewhere).  gen counts the builds that rebuilt the list; the recording
+  // pass after a build writes, for each fluid particle (by slot), vl_n
+  // candidates in vl (the layout CandReader reads): the records of its tile's
+  // block that were binned within the list radius (the search radius plus
+  // 2 sqrt(2) skins, what two particles can close before a rebuild), in the
+  // stencil walk's order, or vl_n == kVlOverflow when there were more than
+  // vl_cap.
   unsigned *gen;           // [1]
   unsigned short *vl;      // [vl_cap * nf], vl_cap a multiple of 8
   unsigned char *vl_n;     // [nf]
@@ -229,9 +231,10 @@ struct CellGrid {
 constexpr int kVlCapMax = 240;  // vl_n is a byte
 constexpr unsigned char kVlOverflow = 255;
 
-// Statistics of a rate pass, zeroed by the cell-list launch before it: pairs
-// (i < j) counted from the i side, and the largest in-radius neighbour count
-// of a fluid particle.
+// Statistics of a rate pass: pairs (i < j) counted from the i side, and the
+// largest in-radius neighbour count of a fluid particle.  Zeroed by the
+// cell-list launch before a tiled pass, published by the launch of a step that
+// streams.
 struct PassStats {
   unsigned long long *niac;
   int *max_nb;
@@ -283,9 +286,10 @@ uph_status launch_cell_build(const DevParams &P, const double *x, const double *
 // the caller then swaps the two.  D must hold the same particle constants
 // (mass, type, reference index, sponge factor) as S, and the walls' fields;
 // where walls move the pass also moves D's walls: walls == 1
-// to this step's time, *d_itime dt (where S's walls are), walls == 2 to the
-// next step's, (*d_itime + 1) dt.  enabled == 0: the pass writes only the
-// rates, into S.
+// to this step's time (where S's walls are), walls == 2 to the next step's.
+// This step's time is *d_itime dt in a tiled pass, behind the list launch that
+// counted the step, and (*d_itime + 1) dt in a launch that streams, which
+// counts it at its end.  enabled == 0: the pass writes only the rates, into S.
 struct StepOut {
   SlotArrays D;
   WallTable W;
@@ -346,7 +350,8 @@ void launch_correct(const DevParams &P, const SlotArrays &S, const WallTable &W,
                     int walls_next, unsigned *err, const int *d_itime, cudaStream_t s);
 void launch_refresh_inverse(const DevParams &P, const SlotArrays &S, int first, int count, cudaStream_t s);
 // t = (*d_itime + 1) dt when d_itime is given: the counter holds the steps
-// started (the cell-list launch of each step of uph_sim_step advances it)
+// started (each step of uph_sim_step advances it, by its cell-list launch or
+// at the end of its one launch)
 // and lives on the device so CUDA-graph replays see the right time;
 // else t = t_host
 void launch_wall_motion(const DevParams &P, const SlotArrays &S, const WallTable &W, double t_host,
