@@ -681,9 +681,11 @@ def main():
     cpu = None
     if world == 1 and not args.no_cpu_baseline:
         v, steps, threads, kind, share = cpu_reference_run(r["deck"], budget_s=args.cpu_budget, max_steps=1000)
+        what = "reference solver compiled from its sources; search stand-in for libnabo"
+        if kind == "port":
+            what = "CPU restatement of the reference, one thread"
         cpu = {"value": v, "unit": UNIT, "cores": threads, "kind": kind, "inputbp_share_of_step": share,
-               "sample": f"{steps} leapfrog steps of the same 500k-particle tank on the host "
-                         f"(reference solver compiled from its sources; search stand-in for libnabo)"}
+               "sample": f"{steps} leapfrog steps of the same 500k-particle tank on the host ({what})"}
     kt = {k: {"ms_total": round(v[0], 4), "launches": v[1]} for k, v in r["ktimes"].items() if v[1]}
     line = {
         "metric": METRIC, "value": r["value"], "unit": UNIT, "n_gpus": world, "steps": args.steps,
