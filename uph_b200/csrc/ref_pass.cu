@@ -663,7 +663,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_ref_pass(const DevParams P,
   }
   unsigned my_pairs = 0;
   int my_nb = 0;  // largest in-radius count of this thread's particles
-  ref_tile<kBrute, kKnn>(P, S, G, F, blockIdx.x, smem, my_pairs, my_nb);
+  if (const int tile = pass_tile(G); tile >= 0) ref_tile<kBrute, kKnn>(P, S, G, F, tile, smem, my_pairs, my_nb);
   pass_stats(st, my_pairs, my_nb);
 }
 

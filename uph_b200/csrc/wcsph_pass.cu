@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_wcsph_pass(const DevParams 
   }
   unsigned my_pairs = 0;
   int my_nb = 0;  // largest in-radius count of this thread's particles
-  wc_tile<kBrute, Real>(P, S, G, F, blockIdx.x, smem, my_pairs, my_nb);
+  if (const int tile = pass_tile(G); tile >= 0) wc_tile<kBrute, Real>(P, S, G, F, tile, smem, my_pairs, my_nb);
   pass_stats(st, my_pairs, my_nb);
 }
 
