@@ -469,11 +469,16 @@ bool steps_stream(const DevParams &P)
   return P.knn == 0 && P.nf > 0 && (P.profile != UPH_PROFILE_REF || P.flag_init_simul == 1);
 }
 
-// Whether a lattice has at most knn points in radius, so that the cap cuts few
-// queries (crowded ones).  (A search knows no lattice.)
+// Whether the cap's cut counts a lane a query first (launch_knn_cut): a
+// lattice has at most knn points in radius, so that the cap cuts few queries
+// (crowded ones), and there are enough of them to fill the machine a lane each.
+// us a step at h = 1.3 dx under the cap of 40, a warp a query / a lane: 3,000
+// particles 49 / 51, 6,000 52 / 54, 10,000 54 / 54, 15,000 64 / 60, 30,000 76 /
+// 60, 100,000 160 / 98.  (A search knows no lattice.)
+constexpr int kCountQueries = 10000;
 bool few_in_radius(const uph_sim *s)
 {
-  return !s->search_only && 3.14159 * s->P.r2cut <= s->P.knn * s->P.dx * s->P.dx;
+  return !s->search_only && s->P.nf >= kCountQueries && 3.14159 * s->P.r2cut <= s->P.knn * s->P.dx * s->P.dx;
 }
 
 // Whether a lattice's tiles fit the stream (tile_stream.cuh): the block's

@@ -319,7 +319,8 @@ struct VirtualPoints {
   CellGrid grid;
 };
 // the knn cap's cut of every fluid query (P.kcut_*), from the cell list and
-// the virtual points; few: most queries have at most knn points in radius
+// the virtual points; few: most of many queries have at most knn points in
+// radius
 void launch_knn_cut(const DevParams &P, const SlotArrays &S, const CellGrid &G, const VirtualPoints &V, bool few,
                     cudaStream_t s);
 // Scratch and results of the virtual particles: flags and offsets by
